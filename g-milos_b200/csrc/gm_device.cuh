@@ -179,28 +179,33 @@ struct Jacobi11 {
   double V[S11 ? 2 : 1][S11 ? 144 : 1];
 };
 
-// Warp-private shared memory.
+// Warp-private shared memory: the half-warp solve's space, then the models and
+// what a synthesis touches, then the staged rows.  The wave kernels back only
+// a part of it (a warp's stride in their shared memory): a trial the rows' first
+// 8-row tile, and kernels that leave the solve to the solve kernel nothing
+// before m.
 template <int LPL, int V>
 struct WarpSmem {
   static constexpr int NR = Variant<V>::ROWS;
   static constexpr bool S11 = V == 2;
-  double m[11];          // current (last accepted) model: the reference's initModel
-  double t[11];          // trial model, persistent like the reference's `model`
   static constexpr int NS = Variant<V>::SOLVES;
-  // Jacobi working matrix per damping, double-buffered, in 2x2 blocks of
+  // solve10's space.  Jacobi working matrix per damping, double-buffered, in 2x2 blocks of
   // the upper triangle (solve10's layout: damping h, buffer b at
   // h * kSolveH + b * kSolveB)
   alignas(16) float A[NS == 2 ? 272 : 200];
-  float alpha[68];       // undamped normal matrix, packed upper triangle (55 or 66)
-  float beta[12];
   float vec[NS][2][12];  // rotated beta per damping, double-buffered; a step lands in vec[d][0]
   float cs[NS][18][5], sn[NS][18][5];
+  // from here on: what the wave kernels without their own solve touch
+  alignas(16) double m[11];   // current (last accepted) model: the reference's initModel
+  double t[11];          // trial model, persistent like the reference's `model`
   float ic[NR];          // continuum about which each staged I row is reflected
   double gk[Variant<V>::MAC ? kMaxNl : 1];   // macroturbulence kernel (PSF folded in)
   double gd[Variant<V>::MAC ? kMaxNl : 1];   // its derivative with respect to v_mac
-  double dd[12];         // FP64 step of the 11-term solve
+  double dd[S11 ? 12 : 1];                   // FP64 step of the 11-term solve
   double b11[S11 ? 12 : 1], z11[S11 ? 12 : 1];
   double c11[S11 ? 6 : 1], s11[S11 ? 6 : 1]; // the step's rotations
+  float alpha[68];       // undamped normal matrix, packed upper triangle (55 or 66)
+  float beta[12];
   // staged rows (PSF, macroturbulence, RFs), sharing their space with the
   // 11-term solve's matrices: a trial solves before its synthesis stages
   // any row, the accept half never solves, and the response functions are
@@ -1336,6 +1341,114 @@ __device__ __noinline__ void solve10(WarpSmem<LPL, V>& sm, const SolvePlan& pl, 
   __syncwarp();
 }
 
+// --------------------------------------------------------------- 10x10 solve, one thread each
+// solve10's arithmetic with a whole system in one thread's registers: the
+// same 18 steps on the same 2x2 blocks in the same order, every product and
+// multiply-add written out as solve10's expressions compile (which product
+// of a pair is fused and which is rounded first), so a step's result is that
+// of solve10 bit for bit.  What it saves is lanes: solve10's half-warp forms each angle
+// on 16 lanes where 5 differ, moves every entry through shared memory and
+// waits at a barrier per step; here the relabelling is register naming.
+__device__ __forceinline__ float mul_sub(float a, float b, float c, float d) {   // a b - c d
+  return __fmaf_rn(a, b, -__fmul_rn(c, d));
+}
+__device__ __forceinline__ float mul_add(float a, float b, float c, float d) {   // a b + c d
+  return __fmaf_rn(a, b, __fmul_rn(c, d));
+}
+// position of component i after a step's round-robin relabelling
+__host__ __device__ constexpr int relabel10(int i) {
+  constexpr int pr[10] = {0, 2, 4, 1, 6, 3, 8, 5, 9, 7};
+  return pr[i];
+}
+// packed index of entry (i, j) of the symmetric matrix
+__host__ __device__ constexpr int sym10(int i, int j) { return i <= j ? upk<10>(i, j) : upk<10>(j, i); }
+
+// One step: the angles of the five diagonal blocks (kept at ang[32 p] for
+// the way back), every block rotated and moved, the vector rotated and moved.
+template <bool accurate>
+__device__ __forceinline__ void jacobi_step(float (&A)[55], float (&v)[10], float* ang) {
+  float cs[5], sn[5];
+  const float quarter = (float)(kPi / 4);
+  const float qclamp = __fdividef((float)kPi, 4.f);
+#pragma unroll
+  for (int p = 0; p < 5; ++p) {
+    const float m00 = A[sym10(2 * p, 2 * p)], m01 = A[sym10(2 * p, 2 * p + 1)],
+                m11 = A[sym10(2 * p + 1, 2 * p + 1)];
+    const float num = 2.f * m01, den = m11 - m00;
+    const float arc = accurate ? num / den : __fdividef(num, den);
+    float th = accurate ? atanf(arc) / 2.f : __fdividef(atanf(arc), 2.f);
+    th = fminf(fmaxf(th, -qclamp), qclamp);
+    if (m00 == m11) th = quarter;
+    ang[32 * p] = th;
+    sincos_mode(th, &sn[p], &cs[p], accurate);
+  }
+  float B[55], u[10];
+#pragma unroll
+  for (int p = 0; p < 5; ++p) {
+    const int r0 = 2 * p, r1 = 2 * p + 1;
+    const float cr = cs[p], sr = sn[p];
+    u[relabel10(r0)] = mul_sub(cr, v[r0], sr, v[r1]);
+    u[relabel10(r1)] = mul_add(sr, v[r0], cr, v[r1]);
+#pragma unroll
+    for (int q = p; q < 5; ++q) {
+      const int c0 = 2 * q, c1 = 2 * q + 1;
+      const float cc = cs[q], sc = sn[q];
+      const float m00 = A[sym10(r0, c0)], m01 = A[sym10(r0, c1)], m10 = A[sym10(r1, c0)], m11 = A[sym10(r1, c1)];
+      const float t0 = mul_sub(m00, cr, m10, sr), t1 = mul_add(m10, cr, m00, sr);
+      const float u0 = mul_sub(m01, cr, m11, sr), u1 = mul_add(m11, cr, m01, sr);
+      B[sym10(relabel10(r0), relabel10(c0))] = mul_sub(t0, cc, u0, sc);
+      B[sym10(relabel10(r1), relabel10(c1))] = mul_add(t1, sc, u1, cc);
+      B[sym10(relabel10(r0), relabel10(c1))] = p == q ? 0.f : mul_add(t0, sc, u0, cc);
+      if (p != q) B[sym10(relabel10(r1), relabel10(c0))] = mul_sub(t1, cc, u1, sc);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 55; ++i) A[i] = B[i];
+#pragma unroll
+  for (int i = 0; i < 10; ++i) v[i] = u[i];
+}
+
+// delta (in v) of the damped system A (its diagonal already damped, entries
+// packed as upk<10>) and beta (v on entry).  ang: this lane's column of the
+// warp's kSolveAngles x 32 angles in shared memory; their sines and cosines
+// are taken again on the way back (half the space of keeping both, which
+// decides how many warps an SM holds).
+constexpr int kSolveAngles = 18 * 5;
+template <bool accurate>
+__device__ __forceinline__ void solve10_thread(float (&A)[55], float (&v)[10], float* ang) {
+  constexpr int kUnroll = 3;
+#pragma unroll 1
+  for (int s0 = 0; s0 < 18; s0 += kUnroll)
+#pragma unroll
+    for (int k = 0; k < kUnroll; ++k) jacobi_step<accurate>(A, v, ang + (s0 + k) * 160);
+  float y[10];
+#pragma unroll
+  for (int i = 0; i < 10; ++i) {
+    const float w = A[sym10(i, i)];
+    const float inv = ((double)fabsf(w) > 1e-12) ? (1.f / w) : 0.f;
+    y[i] = v[i] * inv;
+  }
+#pragma unroll 1
+  for (int s0 = 18 - kUnroll; s0 >= 0; s0 -= kUnroll) {
+#pragma unroll
+    for (int k = kUnroll - 1; k >= 0; --k) {
+      float z[10];
+#pragma unroll
+      for (int p = 0; p < 5; ++p) {
+        float sn, cs;
+        sincos_mode(ang[(s0 + k) * 160 + 32 * p], &sn, &cs, accurate);
+        const float y0 = y[relabel10(2 * p)], y1 = y[relabel10(2 * p + 1)];
+        z[2 * p] = mul_add(cs, y0, sn, y1);
+        z[2 * p + 1] = mul_sub(cs, y1, sn, y0);
+      }
+#pragma unroll
+      for (int i = 0; i < 10; ++i) y[i] = z[i];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 10; ++i) v[i] = y[i];
+}
+
 // --------------------------------------------------------------- 11x11 solve (FP64)
 // delta = V diag(1/w) V^T beta for the damped 11x11 normal matrix in double
 // with the |w| <= 1e-12 cut (mil_svd, milosUtils.cu:280-325).  The reference
@@ -1541,33 +1654,43 @@ __device__ __forceinline__ bool solve11_elim(WarpSmem<LPL, V>& sm, float flambda
 // (AplicaDeltaf, milosUtils.cu:93-159, float delta; AplicaDelta, :30-91,
 // double delta for 11 terms), then range checks (check, :160-238).  The
 // filling factor's step is slot 9 of 10 or slot 10 of 11.
-template <int NT, typename T>
-__device__ __forceinline__ void apply_delta_check(const DevCfg& c, const double* m, const T* d,
-                                                  double* t) {
+// fix: the free-parameter flags, an array or a FixMask.
+struct FixMask {
+  uint32_t bits;
+  __device__ __forceinline__ bool operator[](int i) const { return (bits >> i) & 1u; }
+};
+__device__ __forceinline__ FixMask fix_mask(const DevCfg& c) {
+  FixMask f{0u};
+#pragma unroll
+  for (int i = 0; i < 11; ++i) f.bits |= (c.fix[i] ? 1u : 0u) << i;
+  return f;
+}
+template <int NT, typename T, typename F>
+__device__ __forceinline__ void apply_delta_check(const F& fix, const double* m, const T* d, double* t) {
   T aux;
-  if (c.fix[ETA0]) t[ETA0] = m[ETA0] - d[0];
-  if (c.fix[BFLD]) {
+  if (fix[ETA0]) t[ETA0] = m[ETA0] - d[0];
+  if (fix[BFLD]) {
     aux = d[1];
     if (aux < -300) aux = -300; else if (aux > 300) aux = 300;
     t[BFLD] = m[BFLD] - aux;
   }
-  if (c.fix[VLOS]) t[VLOS] = m[VLOS] - d[2];
-  if (c.fix[DOPP]) t[DOPP] = m[DOPP] - d[3];
-  if (c.fix[AA]) t[AA] = m[AA] - d[4];
-  if (c.fix[GM]) {
+  if (fix[VLOS]) t[VLOS] = m[VLOS] - d[2];
+  if (fix[DOPP]) t[DOPP] = m[DOPP] - d[3];
+  if (fix[AA]) t[AA] = m[AA] - d[4];
+  if (fix[GM]) {
     aux = d[5];
     if (aux < -30) aux = -30; else if (aux > 30) aux = 30;
     t[GM] = m[GM] - aux;
   }
-  if (c.fix[AZ]) {
+  if (fix[AZ]) {
     aux = d[6];
     if (aux < -30) aux = -30; else if (aux > 30) aux = 30;
     t[AZ] = m[AZ] - aux;
   }
-  if (c.fix[S0]) t[S0] = m[S0] - d[7];
-  if (c.fix[S1]) t[S1] = m[S1] - d[8];
-  if (c.fix[MAC]) t[MAC] = m[MAC] - d[9];
-  if (c.fix[ALFA]) t[ALFA] = m[ALFA] - d[NT == 11 ? 10 : 9];
+  if (fix[S0]) t[S0] = m[S0] - d[7];
+  if (fix[S1]) t[S1] = m[S1] - d[8];
+  if (fix[MAC]) t[MAC] = m[MAC] - d[9];
+  if (fix[ALFA]) t[ALFA] = m[ALFA] - d[NT == 11 ? 10 : 9];
   if (t[BFLD] < 0) { t[BFLD] = -t[BFLD]; t[GM] = 180.0 - t[GM]; }
   if (t[BFLD] > 5000) t[BFLD] = 5000;
   if (t[GM] < 0) t[GM] = -t[GM];

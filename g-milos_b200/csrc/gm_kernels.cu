@@ -134,10 +134,10 @@ invert_kernel(const DevCfg c, const InvertArgs a) {
             else solve10<LPL, V, false>(sm, plan, flambda, flambda * 10.f * pbf, lane);
           }
           solved = !reuse;
-          if (lane == 0) apply_delta_check<10>(c, sm.m, sm.vec[reuse ? 1 : 0][0], sm.t);
+          if (lane == 0) apply_delta_check<10>(c.fix, sm.m, sm.vec[reuse ? 1 : 0][0], sm.t);
         } else {
           if (!solve11_elim<LPL, V>(sm, flambda, lane)) solve11<LPL, V>(sm, plan11, flambda, lane);
-          if (lane == 0) apply_delta_check<11>(c, sm.m, sm.dd, sm.t);
+          if (lane == 0) apply_delta_check<11>(c.fix, sm.m, sm.dd, sm.t);
         }
         __syncwarp();
       }
@@ -232,10 +232,11 @@ invert_kernel(const DevCfg c, const InvertArgs a) {
 // pixels still iterating -- the step solve, the step limits, the trial
 // synthesis with PSF and stray light, chi2 and the damping schedule -- then
 // accept_kernel over the pixels whose trial was accepted: response
-// functions, their PSF and the normal equations.  Each kernel executes
-// about a third of invert_kernel's code, so the warps of an SM share one hot
-// instruction working set, and each has its own register budget (at nl <=
-// 32 the trial half runs 28 warps per SM, the accept half 20).  A pixel's
+// functions, their PSF and the normal equations -- and, in chunks large enough
+// (solve_apart), solve_kernel for the next wave's steps, which trial_kernel
+// else makes itself.  Each kernel executes a third or less of
+// invert_kernel's code, so the warps of an SM share one hot instruction
+// working set, and each has its own register budget.  A pixel's
 // LM state lives in a PixLM record between the kernels; the per-lane Voigt
 // and Zeeman terms, angles and profiles of an accepted trial reach the
 // accept kernel through a staging row block, so nothing is recomputed: each
@@ -243,24 +244,38 @@ invert_kernel(const DevCfg c, const InvertArgs a) {
 // kernels, the multiply-adds the compiler fuses differ, so results agree
 // with invert_kernel's to rounding, not bit for bit).
 
-// Resident blocks per SM: registers for the 10-term variants; the 11-term
-// variant's FP64 Jacobi matrices make shared memory the limit.
+// Resident blocks per SM.  Trials whose step the solve kernel makes (SK) spill
+// nothing at 96 registers, and 20 warps per SM beat more: the 1024 x 1024
+// cube of 30 samples takes 242, 246, 258, 262 ms at 5, 6, 7, 8 blocks (20 to 32
+// warps), 251 ms at 4.  With the solve in the trial kernel 28 warps are best.
+// At 33 to 64 samples 8 to 12 blocks of 2 warps measure the same to 0.5 %.
+// Accept half: 243 ms at 5 blocks, 246 at 4, 248 at 6.
+template <int LPL, int V, bool SK>
+constexpr int trial_min_blocks() { return LPL == 1 ? (V != 2 && !SK ? 7 : 5) : (V == 2 ? 8 : 10); }
 template <int LPL, int V>
-constexpr int trial_min_blocks() { return V == 2 ? (LPL == 1 ? 5 : 8) : (LPL == 1 ? 7 : 10); }
-template <int LPL, int V>
-constexpr int accept_min_blocks() { return V == 2 ? (LPL == 1 ? 5 : 5) : 5; }
+constexpr int accept_min_blocks() { return 5; }
 
-// The trial half touches the warp's shared memory only up to the first
-// 8-row tile of staged rows (the synthesis PSF stages rows 0-3) -- or, in
-// the 11-term variant, up to the end of the solve's matrices that share the
-// rows' space -- so its warps are packed at that stride: half the
-// footprint, more warps per SM.
-template <int LPL, int V>
+// The part of the warp's shared memory the wave kernels back.  The trial half
+// touches it only up to the first 8-row tile of staged rows (the synthesis PSF
+// stages rows 0-3) -- or, in the 11-term variant, up to the end of the solve's
+// matrices that share the rows' space -- so its warps are packed at that
+// stride.  SK: the solve kernel makes the steps, so solve10's space, which
+// comes first, is not backed.
+template <int LPL, int V, bool SK>
+__host__ __device__ constexpr size_t wave_smem_begin() {
+  using WS = WarpSmem<LPL, V>;
+  return SK ? offsetof(WS, m) : 0;
+}
+template <int LPL, int V, bool SK>
 __host__ __device__ constexpr size_t trial_warp_bytes() {
   using WS = WarpSmem<LPL, V>;
   constexpr size_t tile = 8 * row_pitch<LPL>() * sizeof(float);
   constexpr size_t solve = V == 2 ? sizeof(Jacobi11<true>) : 0;   // the 11-term solve's matrices
-  return (offsetof(WS, rows) + (tile > solve ? tile : solve) + 15) & ~(size_t)15;
+  return ((offsetof(WS, rows) + (tile > solve ? tile : solve) + 15) & ~(size_t)15) - wave_smem_begin<LPL, V, SK>();
+}
+template <int LPL, int V>
+__host__ __device__ constexpr size_t accept_warp_bytes() {
+  return sizeof(WarpSmem<LPL, V>) - wave_smem_begin<LPL, V, true>();
 }
 template <int LPL, int V>
 constexpr bool xrows_follow_rows() {
@@ -270,10 +285,17 @@ constexpr bool xrows_follow_rows() {
 static_assert(xrows_follow_rows<1, 0>() && xrows_follow_rows<1, 1>() && xrows_follow_rows<1, 2>() &&
                   xrows_follow_rows<2, 0>() && xrows_follow_rows<2, 1>() && xrows_follow_rows<2, 2>(),
               "the operand rows must follow the staged rows");
-template <int LPL, int V>
+template <int LPL, int V, bool SK>
 __device__ __forceinline__ WarpSmem<LPL, V>& trial_smem() {
   return *reinterpret_cast<WarpSmem<LPL, V>*>(gm_dyn_smem + tap_bytes<LPL>() +
-                                               (threadIdx.x >> 5) * trial_warp_bytes<LPL, V>());
+                                               (threadIdx.x >> 5) * trial_warp_bytes<LPL, V, SK>() -
+                                               wave_smem_begin<LPL, V, SK>());
+}
+template <int LPL, int V>
+__device__ __forceinline__ WarpSmem<LPL, V>& accept_smem() {
+  return *reinterpret_cast<WarpSmem<LPL, V>*>(gm_dyn_smem + tap_bytes<LPL>() +
+                                               (threadIdx.x >> 5) * accept_warp_bytes<LPL, V>() -
+                                               wave_smem_begin<LPL, V, true>());
 }
 
 // Staged rows of an accepted trial (one float per lane each): per sample
@@ -400,14 +422,15 @@ constexpr int wave_warps() { return MG ? 1 : warps_per_block<LPL>(); }
 // One trial of every pixel in the wave's active list (wave 0: the start
 // models, every pixel of the chunk).  The body is invert_kernel's loop
 // body from the solve to the damping schedule (milosUtils.cu:630-700).
-template <int LPL, int V, bool MG>
+template <int LPL, int V, bool MG, bool SK>
 __global__ void __launch_bounds__(wave_warps<LPL, MG>() * 32,
-                                  trial_min_blocks<LPL, V>() * warps_per_block<LPL>() / wave_warps<LPL, MG>())
+                                  trial_min_blocks<LPL, V, SK>() * warps_per_block<LPL>() / wave_warps<LPL, MG>())
 trial_kernel(const DevCfg c0, const InvertArgs a, const WaveArgs w, int wave, const MultiGrid mg) {
   constexpr int NS = Variant<V>::SOLVES, NT = Variant<V>::NT, NA = NT * (NT + 1) / 2;
+  constexpr bool SECOND = NT == 10 && (SK || NS == 2);   // two dampings solved at once
   const int lane = threadIdx.x & 31;
   if constexpr (!MG) load_taps<LPL>(c0);
-  WarpSmem<LPL, V>& sm = trial_smem<LPL, V>();
+  WarpSmem<LPL, V>& sm = trial_smem<LPL, V, SK>();
   for (int i = lane; i < 8 * row_pitch<LPL>(); i += 32) (&sm.rows[0][0])[i] = 0.f;
   __syncwarp();
   int nl = c0.nl;
@@ -430,19 +453,23 @@ trial_kernel(const DevCfg c0, const InvertArgs a, const WaveArgs w, int wave, co
       for (int s = 0; s < 4; ++s) slg[k][s] = 0.f;
   }
   int cur = -1;   // grid whose constants are loaded (ragged batches)
-  const SolvePlan plan = g_solve_plans[NS - 1].lane[lane];
+  SolvePlan plan;
   Solve11Plan plan11;
+  if constexpr (NT == 10 && !SK) plan = g_solve_plans[NS - 1].lane[lane];
   if constexpr (NT == 11) plan11 = make_solve11_plan(lane);
-  const uint32_t n = wave == 0 ? (uint32_t)a.npix : w.cnt[wave - 1].n_next;
+  const uint32_t nsolve = wave == 0 ? (uint32_t)a.npix : w.cnt[wave - 1].n_solve;
+  const uint32_t n = wave == 0 ? nsolve : nsolve + w.cnt[wave - 1].n_reuse;
   const uint32_t* in = (wave & 1) ? w.act1 : w.act0;
   uint32_t* next = (wave & 1) ? w.act0 : w.act1;
+  // the wave's accept kernel starts after this one, the last wave's has ended
+  if (blockIdx.x == 0 && threadIdx.x == 0) *w.cur_acc = 0u;
   unsigned long long my_iter = 0, my_acc = 0;
   while (true) {
     uint32_t j = 0;
     if (lane == 0) j = atomicAdd(&w.cnt[wave].cur_trial, 1u);
     j = __shfl_sync(kFull, j, 0);
     if (j >= n) break;
-    const uint32_t pix = wave == 0 ? j : in[j];
+    const uint32_t pix = wave == 0 ? j : in[j < nsolve ? j : w.cap - 1 - (j - nsolve)];
     const DevCfg* cp = nullptr;
     if constexpr (MG) {
       const int gi = mg.grid[pix];
@@ -474,10 +501,10 @@ trial_kernel(const DevCfg c0, const InvertArgs a, const WaveArgs w, int wave, co
       iter = acc = 0;
       __syncwarp();
     } else {
-      const bool reuse = NS == 2 && (P.flags & 1u);
+      const bool reuse = SECOND && (P.flags & 1u);
       if (lane < 11) {
         sm.m[lane] = P.m[lane];
-        sm.t[lane] = P.t[lane];
+        sm.t[lane] = P.t[lane];   // SK: the solve kernel's trial model
       }
       flambda = P.flambda;
       pbf = P.pbf;
@@ -486,22 +513,24 @@ trial_kernel(const DevCfg c0, const InvertArgs a, const WaveArgs w, int wave, co
       iter = P.iter;
       acc = P.acc;
       st = P.st;
-      if (reuse) {
-        if (lane < 10) sm.vec[1][0][lane] = P.vnext[lane];
-      } else {
-        for (int i = lane; i < NA; i += 32) sm.alpha[i] = P.alpha[i];
-        if (lane < NT) sm.beta[lane] = P.beta[lane];
-      }
-      __syncwarp();
-      if constexpr (NT == 11) {
-        if (!solve11_elim<LPL, V>(sm, flambda, lane)) solve11<LPL, V>(sm, plan11, flambda, lane);
-        if (lane == 0) apply_delta_check<11>(c, sm.m, sm.dd, sm.t);
-      } else {
-        if (!reuse) {
-          if (c.numerics) solve10<LPL, V, true>(sm, plan, flambda, flambda * 10.f * pbf, lane);
-          else solve10<LPL, V, false>(sm, plan, flambda, flambda * 10.f * pbf, lane);
+      if constexpr (!SK) {
+        if (reuse) {
+          if (lane < 10) sm.vec[NS - 1][0][lane] = P.vnext[lane];
+        } else {
+          for (int i = lane; i < NA; i += 32) sm.alpha[i] = P.alpha[i];
+          if (lane < NT) sm.beta[lane] = P.beta[lane];
         }
-        if (lane == 0) apply_delta_check<10>(c, sm.m, sm.vec[reuse ? 1 : 0][0], sm.t);
+        __syncwarp();
+        if constexpr (NT == 11) {
+          if (!solve11_elim<LPL, V>(sm, flambda, lane)) solve11<LPL, V>(sm, plan11, flambda, lane);
+          if (lane == 0) apply_delta_check<11>(c.fix, sm.m, sm.dd, sm.t);
+        } else {
+          if (!reuse) {
+            if (c.numerics) solve10<LPL, V, true>(sm, plan, flambda, flambda * 10.f * pbf, lane);
+            else solve10<LPL, V, false>(sm, plan, flambda, flambda * 10.f * pbf, lane);
+          }
+          if (lane == 0) apply_delta_check<10>(c.fix, sm.m, sm.vec[reuse ? NS - 1 : 0][0], sm.t);
+        }
       }
       solved = !reuse;
       __syncwarp();
@@ -538,7 +567,7 @@ trial_kernel(const DevCfg c0, const InvertArgs a, const WaveArgs w, int wave, co
         st |= GM_PIX_LAMBDA_EXIT;
       }
       ++iter;
-      have_next = NS == 2 && !accept && solved;
+      have_next = SECOND && !accept && solved;
       if (c.logclambda) pbf = log10f(chisqr) / log10f(chisqr0);
       if (accept) ochisqr = chisqr;
     }
@@ -551,10 +580,10 @@ trial_kernel(const DevCfg c0, const InvertArgs a, const WaveArgs w, int wave, co
       my_acc += acc;
     } else {
       if (lane < 11) {
-        P.m[lane] = sm.m[lane];
-        P.t[lane] = sm.t[lane];
+        if (accept) P.m[lane] = sm.m[lane];
+        if (!SK || wave == 0) P.t[lane] = sm.t[lane];   // else the solve kernel's, as read
       }
-      if (NS == 2 && solved && lane < 10) P.vnext[lane] = sm.vec[NS - 1][0][lane];
+      if (!SK && NS == 2 && solved && lane < 10) P.vnext[lane] = sm.vec[NS - 1][0][lane];
       uint32_t slot = 0, aslot = 0;
       if (lane == 0) {
         P.flambda = flambda;
@@ -565,7 +594,7 @@ trial_kernel(const DevCfg c0, const InvertArgs a, const WaveArgs w, int wave, co
         P.acc = acc;
         P.st = st;
         P.flags = have_next ? 1u : 0u;
-        slot = atomicAdd(&w.cnt[wave].n_next, 1u);
+        slot = have_next ? w.cap - 1 - atomicAdd(&w.cnt[wave].n_reuse, 1u) : atomicAdd(&w.cnt[wave].n_solve, 1u);
         if (accept) aslot = atomicAdd(&w.cnt[wave].n_acc, 1u);
       }
       slot = __shfl_sync(kFull, slot, 0);
@@ -584,6 +613,98 @@ trial_kernel(const DevCfg c0, const InvertArgs a, const WaveArgs w, int wave, co
   }
 }
 
+// The next trial models of the 10-term variants, between a wave's accept
+// kernel and the next wave's trial kernel: one thread per 10x10 system.  A
+// pixel whose normal equations are new (its trial was accepted), or whose
+// second damping is used up, is solved for the damping of its next trial and
+// for the one a rejection of that moves to, by the threads l and l + 16 of a
+// warp; a pixel that holds its next step already only takes it.  The step
+// limits and range checks (apply_delta_check) follow in the same thread.
+//
+// Bound by instruction issue (59 % of cycles, FMA pipe 45 %): about 430
+// instructions a step for 32 systems, where the half-warp solve10 takes about
+// 100 for two.  16 warps per SM of 128 registers and 11.5 KB of angles hold a
+// system in registers; the sines and cosines kept as well, in local memory,
+// made it 68 us a wave instead of 38 (65 536 pixels, average over the waves),
+// and the same solve at the end of the accept kernel, by the warp that
+// completes 16 pixels, 276 ms instead of 242 (1024 x 1024 cube, 297 ms with
+// solve10 in the trial kernel): three kinds of code in one kernel miss the
+// instruction cache.
+constexpr int kSolveThreads = 64, kSolvePix = 16, kSolveBlocks = 8;
+template <bool ACC>
+__global__ void __launch_bounds__(kSolveThreads, kSolveBlocks)
+solve_kernel(const DevCfg c, const WaveArgs w, int wave) {
+  // a pixel's alpha and beta in 17 16-byte vectors; the odd pitch keeps the
+  // lanes' reads in distinct banks.  The angles take the same space.
+  constexpr int NV = 17, PITCH = 69;
+  __shared__ float space[kSolveThreads / 32][kSolveAngles * 32];
+  static_assert(kSolvePix * PITCH <= kSolveAngles * 32 && offsetof(PixLM, beta) == offsetof(PixLM, alpha) + 68 * 4,
+                "the tile shares the angles' space");
+  const int lane = threadIdx.x & 31, px = lane & (kSolvePix - 1), h = lane / kSolvePix;
+  float* sw = space[threadIdx.x >> 5];
+  const uint32_t* list = (wave & 1) ? w.act0 : w.act1;
+  const uint32_t ns = w.cnt[wave].n_solve, nr = w.cnt[wave].n_reuse;
+  const uint32_t tid = blockIdx.x * kSolveThreads + threadIdx.x, nth = gridDim.x * kSolveThreads;
+  for (uint32_t i = tid; i < nr; i += nth) {
+    PixLM& P = w.state[list[w.cap - 1 - i]];
+    double t[11];
+#pragma unroll
+    for (int k = 0; k < 11; ++k) t[k] = P.t[k];
+    apply_delta_check<10>(c.fix, P.m, P.vnext, t);
+#pragma unroll
+    for (int k = 0; k < 11; ++k) P.t[k] = t[k];
+  }
+  for (uint32_t g = tid / 32; g * kSolvePix < ns; g += nth / 32) {
+    const uint32_t i = g * kSolvePix + px;
+    const bool mine = i < ns;
+    const uint32_t pix = list[mine ? i : ns - 1];
+    PixLM& P = w.state[pix];
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < (kSolvePix * NV + 31) / 32; ++k) {
+      const int idx = k * 32 + lane, p = idx / NV, e = idx - p * NV;
+      const PixLM& Q = w.state[__shfl_sync(kFull, pix, p & (kSolvePix - 1))];
+      if (idx < kSolvePix * NV) {
+        const float4 x = reinterpret_cast<const float4*>(e < 14 ? Q.alpha + 4 * e : Q.beta + 4 * (e - 14))[0];
+        float* d = sw + p * PITCH + 4 * e;
+        d[0] = x.x;
+        d[1] = x.y;
+        d[2] = x.z;
+        d[3] = x.w;
+      }
+    }
+    __syncwarp();
+    const float flambda = h ? P.flambda * 10.f * P.pbf : P.flambda;
+    // damped matrix (diagonal x (1 + lambda), milosUtils.cu:648-652)
+    const double damp = 1.0 + (double)flambda;
+    float A[55], v[10];
+#pragma unroll
+    for (int r = 0; r < 10; ++r)
+#pragma unroll
+      for (int q = r; q < 10; ++q) {
+        const float x = sw[px * PITCH + upk<10>(r, q)];
+        A[upk<10>(r, q)] = r == q ? (float)((double)x * damp) : x;
+      }
+#pragma unroll
+    for (int k = 0; k < 10; ++k) v[k] = sw[px * PITCH + 56 + k];
+    __syncwarp();   // the tile has been read
+    solve10_thread<ACC>(A, v, sw + lane);
+    if (mine) {
+      if (h) {
+#pragma unroll
+        for (int k = 0; k < 10; ++k) P.vnext[k] = v[k];
+      } else {
+        double t[11];
+#pragma unroll
+        for (int k = 0; k < 11; ++k) t[k] = P.t[k];
+        apply_delta_check<10>(c.fix, P.m, v, t);
+#pragma unroll
+        for (int k = 0; k < 11; ++k) P.t[k] = t[k];
+      }
+    }
+  }
+}
+
 // Response functions and normal equations of every pixel whose trial of
 // this wave was accepted (the accept branch of invert_kernel's loop).
 template <int LPL, int V, bool MG>
@@ -591,7 +712,7 @@ __global__ void __launch_bounds__(wave_warps<LPL, MG>() * 32,
                                   accept_min_blocks<LPL, V>() * warps_per_block<LPL>() / wave_warps<LPL, MG>())
 accept_kernel(const DevCfg c0, const InvertArgs a, const WaveArgs w, int wave, const MultiGrid mg) {
   const int lane = threadIdx.x & 31;
-  WarpSmem<LPL, V>& sm = warp_smem<LPL, V>();
+  WarpSmem<LPL, V>& sm = accept_smem<LPL, V>();
   if constexpr (!MG) {
     load_taps<LPL>(c0);
     init_rows<LPL, V>(c0, sm, lane);
@@ -619,7 +740,7 @@ accept_kernel(const DevCfg c0, const InvertArgs a, const WaveArgs w, int wave, c
   const bool alpha_mixed = wave > 0 && c0.quirks;
   while (true) {
     uint32_t j = 0;
-    if (lane == 0) j = atomicAdd(&w.cnt[wave].cur_acc, 1u);
+    if (lane == 0) j = atomicAdd(w.cur_acc, 1u);
     j = __shfl_sync(kFull, j, 0);
     if (j >= n) break;
     const uint32_t pix = w.accl[j];
@@ -999,9 +1120,12 @@ constexpr size_t smem_bytes() { return tap_bytes<LPL>() + sizeof(WarpSmem<LPL, V
 constexpr size_t kSmemPerSm = 228 * 1024;
 template <int LPL, int V>
 constexpr bool wave_blocks_fit() {
-  return (tap_bytes<LPL>() + trial_warp_bytes<LPL, V>() * warps_per_block<LPL>() + 1024) *
-                 trial_min_blocks<LPL, V>() <= kSmemPerSm &&
-         (smem_bytes<LPL, V>() + 1024) * accept_min_blocks<LPL, V>() <= kSmemPerSm;
+  return (tap_bytes<LPL>() + trial_warp_bytes<LPL, V, false>() * warps_per_block<LPL>() + 1024) *
+                 trial_min_blocks<LPL, V, false>() <= kSmemPerSm &&
+         (tap_bytes<LPL>() + trial_warp_bytes<LPL, V, true>() * warps_per_block<LPL>() + 1024) *
+                 trial_min_blocks<LPL, V, true>() <= kSmemPerSm &&
+         (tap_bytes<LPL>() + accept_warp_bytes<LPL, V>() * warps_per_block<LPL>() + 1024) *
+                 accept_min_blocks<LPL, V>() <= kSmemPerSm;
 }
 static_assert(wave_blocks_fit<1, 0>() && wave_blocks_fit<1, 1>() && wave_blocks_fit<1, 2>(), "nl <= 32");
 static_assert(wave_blocks_fit<2, 0>() && wave_blocks_fit<2, 1>() && wave_blocks_fit<2, 2>(), "nl <= 64");
@@ -1082,6 +1206,9 @@ WaveBuffers wave_buffers(void* base, int nl, int miter, int64_t chunk) {
   b.w.act0 = reinterpret_cast<uint32_t*>(p);
   b.w.act1 = b.w.act0 + chunk;
   b.w.accl = b.w.act1 + chunk;
+  b.w.cap = (uint32_t)chunk;
+  // the counters' rounding to 256 bytes leaves at least 16 of the 256 spare bytes
+  b.w.cur_acc = b.w.accl + chunk;
   return b;
 }
 
@@ -1091,54 +1218,76 @@ bool waves_cover(const DevCfg& cfg, const InvertArgs& a) {
 
 // Shared memory of the wave kernels: the block's taps and its warps' blocks
 // (the trial kernel packs its warps at trial_warp_bytes).
+template <int LPL, int V, bool MG, bool SK>
+constexpr size_t wave_trial_smem() {
+  return tap_bytes<LPL>() + trial_warp_bytes<LPL, V, SK>() * wave_warps<LPL, MG>();
+}
 template <int LPL, int V, bool MG>
-constexpr size_t wave_trial_smem() { return tap_bytes<LPL>() + trial_warp_bytes<LPL, V>() * wave_warps<LPL, MG>(); }
-template <int LPL, int V, bool MG>
-constexpr size_t wave_accept_smem() { return tap_bytes<LPL>() + sizeof(WarpSmem<LPL, V>) * wave_warps<LPL, MG>(); }
+constexpr size_t wave_accept_smem() { return tap_bytes<LPL>() + accept_warp_bytes<LPL, V>() * wave_warps<LPL, MG>(); }
 
 // Attributes of both wave kernels and their resident blocks per SM.
-template <int LPL, int V, bool MG>
+template <int LPL, int V, bool MG, bool SK>
 cudaError_t wave_occupancy(int* bt, int* ba) {
-  const size_t tsmem = wave_trial_smem<LPL, V, MG>(), smem = wave_accept_smem<LPL, V, MG>();
+  const size_t tsmem = wave_trial_smem<LPL, V, MG, SK>(), smem = wave_accept_smem<LPL, V, MG>();
   cudaError_t e =
-      cudaFuncSetAttribute(trial_kernel<LPL, V, MG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem);
+      cudaFuncSetAttribute(trial_kernel<LPL, V, MG, SK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(accept_kernel<LPL, V, MG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const int threads = wave_warps<LPL, MG>() * 32;
   *bt = *ba = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(bt, trial_kernel<LPL, V, MG>, threads, tsmem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(bt, trial_kernel<LPL, V, MG, SK>, threads, tsmem);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(ba, accept_kernel<LPL, V, MG>, threads, smem);
   return (*bt < 1 || *ba < 1) ? cudaErrorInvalidConfiguration : cudaSuccess;
 }
 
 // The waves of one chunk: a pre-zeroed counter block, then per wave the
-// trial kernel over the pixels still iterating and the accept kernel over
-// those accepted.
-template <int LPL, int V, bool MG>
+// trial kernel over the pixels still iterating, the accept kernel over those
+// accepted and (SK) the solve kernel over those whose next step is not known.
+template <int LPL, int V, bool MG, bool SK>
 cudaError_t run_waves(const DevCfg& dc, const InvertArgs& c, const WaveBuffers& b, const MultiGrid& mg, int gt,
-                      int ga, cudaStream_t s, int* count) {
+                      int ga, int sms, cudaStream_t s, int* count) {
   const int waves = 1 + (dc.miter > 1 ? dc.miter : 1);
   const int threads = wave_warps<LPL, MG>() * 32;
   cudaError_t e = cudaMemsetAsync(b.w.cnt, 0, sizeof(WaveCounters) * (size_t)waves, s);
   if (e != cudaSuccess) return e;
+  // blocks of the solve kernel: every resident slot, or as many as the chunk can need
+  constexpr int per = kSolvePix * kSolveThreads / 32;
+  const int64_t sneed = (c.npix + per - 1) / per, smost = kSolveBlocks * (int64_t)sms;
+  const int gs = (int)(sneed < smost ? sneed : smost);
   for (int wv = 0; wv < waves; ++wv) {
-    trial_kernel<LPL, V, MG><<<gt, threads, wave_trial_smem<LPL, V, MG>(), s>>>(dc, c, b.w, wv, mg);
+    trial_kernel<LPL, V, MG, SK><<<gt, threads, wave_trial_smem<LPL, V, MG, SK>(), s>>>(dc, c, b.w, wv, mg);
     ++*count;
     // the last wave's pixels all stop: nothing to accept
     if (wv + 1 < waves) {
       accept_kernel<LPL, V, MG><<<ga, threads, wave_accept_smem<LPL, V, MG>(), s>>>(dc, c, b.w, wv, mg);
       ++*count;
+      if constexpr (SK) {
+        if (dc.numerics) solve_kernel<true><<<gs, kSolveThreads, 0, s>>>(dc, b.w, wv);
+        else solve_kernel<false><<<gs, kSolveThreads, 0, s>>>(dc, b.w, wv);
+        ++*count;
+      }
     }
   }
   return cudaGetLastError();
 }
 
-template <int LPL, int V>
+// Whether the solve kernel makes the steps of a chunk of n pixels (10 terms;
+// the results are those of the solve in the trial kernel bit for bit).  Its
+// launch pays from about 8000 pixels on: 30 samples and a PSF take 2.87 ms
+// against 2.76 with the solve in the trial kernel at 4096 pixels, 5.42
+// against 5.85 at 16 384, 9.15 against 10.53 at 32 768, 16.6 against 19.8 at
+// 65 536.  Smaller chunks than kSolveApartMin keep two launches a wave, the
+// count gm_stats reports for the smallest calls on these kernels.
+constexpr int64_t kSolveApartMin = 24576;
+template <int V>
+constexpr bool solve_apart(int64_t n) { return V != 2 && n >= kSolveApartMin; }
+
+template <int LPL, int V, bool SK>
 cudaError_t launch_waves_t(const DevCfg& cfg, const InvertArgs& a, const WaveBuffers& b, cudaStream_t s,
                            int* launches) {
   int dev = 0, sms = 0, bt = 0, ba = 0;
-  cudaError_t e = wave_occupancy<LPL, V, false>(&bt, &ba);
+  cudaError_t e = wave_occupancy<LPL, V, false, SK>(&bt, &ba);
   if (e != cudaSuccess) return e;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1150,7 +1299,7 @@ cudaError_t launch_waves_t(const DevCfg& cfg, const InvertArgs& a, const WaveBuf
     const int64_t need = (n + warps_per_block<LPL>() - 1) / warps_per_block<LPL>();
     const int gt = (int)(need < (int64_t)bt * sms ? need : (int64_t)bt * sms);
     const int ga = (int)(need < (int64_t)ba * sms ? need : (int64_t)ba * sms);
-    e = run_waves<LPL, V, false>(dc, c, b, MultiGrid{}, gt, ga, s, &count);
+    e = run_waves<LPL, V, false, SK>(dc, c, b, MultiGrid{}, gt, ga, sms, s, &count);
     if (e != cudaSuccess) return e;
   }
   if (launches) *launches = count;
@@ -1164,7 +1313,8 @@ template <int LPL, int V>
 cudaError_t launch_waves_mg_t(const DevCfg& cfg, const MultiGrid& mg, const InvertArgs& a, const WaveBuffers& b,
                               int cap_t, int cap_a, cudaStream_t s, int* launches) {
   int dev = 0, sms = 0, bt = 0, ba = 0;
-  cudaError_t e = wave_occupancy<LPL, V, true>(&bt, &ba);
+  constexpr bool SK = V != 2;
+  cudaError_t e = wave_occupancy<LPL, V, true, SK>(&bt, &ba);
   if (e != cudaSuccess) return e;
   if (cap_t > 0 && cap_t < bt) bt = cap_t;
   if (cap_a > 0 && cap_a < ba) ba = cap_a;
@@ -1181,7 +1331,7 @@ cudaError_t launch_waves_mg_t(const DevCfg& cfg, const MultiGrid& mg, const Inve
     m.off = mg.off + first;
     const int gt = (int)(n < (int64_t)bt * sms ? n : (int64_t)bt * sms);
     const int ga = (int)(n < (int64_t)ba * sms ? n : (int64_t)ba * sms);
-    e = run_waves<LPL, V, true>(cfg, c, b, m, gt, ga, s, &count);
+    e = run_waves<LPL, V, true, SK>(cfg, c, b, m, gt, ga, sms, s, &count);
     if (e != cudaSuccess) return e;
   }
   if (launches) *launches = count;
@@ -1208,12 +1358,22 @@ void waves_mg_occupancy(const DevCfg& cfg, int* bt, int* ba) {
   const int v = kernel_variant(cfg, false);
   cudaError_t e;
   if (cfg.nl <= 32)
-    e = v == 0 ? wave_occupancy<1, 0, true>(bt, ba) : v == 1 ? wave_occupancy<1, 1, true>(bt, ba)
-                                                             : wave_occupancy<1, 2, true>(bt, ba);
+    e = v == 0 ? wave_occupancy<1, 0, true, true>(bt, ba) : v == 1 ? wave_occupancy<1, 1, true, true>(bt, ba)
+                                                             : wave_occupancy<1, 2, true, false>(bt, ba);
   else
-    e = v == 0 ? wave_occupancy<2, 0, true>(bt, ba) : v == 1 ? wave_occupancy<2, 1, true>(bt, ba)
-                                                             : wave_occupancy<2, 2, true>(bt, ba);
+    e = v == 0 ? wave_occupancy<2, 0, true, true>(bt, ba) : v == 1 ? wave_occupancy<2, 1, true, true>(bt, ba)
+                                                             : wave_occupancy<2, 2, true, false>(bt, ba);
   if (e != cudaSuccess) *bt = *ba = 0;
+}
+
+template <int LPL, int V>
+cudaError_t launch_waves_v(const DevCfg& cfg, const InvertArgs& a, const WaveBuffers& b, cudaStream_t s,
+                           int* launches) {
+  if constexpr (V != 2) {
+    if (solve_apart<V>(a.npix < b.chunk ? a.npix : b.chunk))
+      return launch_waves_t<LPL, V, true>(cfg, a, b, s, launches);
+  }
+  return launch_waves_t<LPL, V, false>(cfg, a, b, s, launches);
 }
 
 cudaError_t launch_invert_waves(const DevCfg& cfg, const InvertArgs& a, const WaveBuffers& b, cudaStream_t s,
@@ -1221,13 +1381,13 @@ cudaError_t launch_invert_waves(const DevCfg& cfg, const InvertArgs& a, const Wa
   if (!waves_cover(cfg, a) || b.chunk < 1 || b.chunk > 0x7fffffff) return cudaErrorInvalidValue;
   const int v = kernel_variant(cfg, a.init_models != nullptr && !a.init_status);
   if (cfg.nl <= 32) {
-    if (v == 0) return launch_waves_t<1, 0>(cfg, a, b, s, launches);
-    if (v == 1) return launch_waves_t<1, 1>(cfg, a, b, s, launches);
-    return launch_waves_t<1, 2>(cfg, a, b, s, launches);
+    if (v == 0) return launch_waves_v<1, 0>(cfg, a, b, s, launches);
+    if (v == 1) return launch_waves_v<1, 1>(cfg, a, b, s, launches);
+    return launch_waves_v<1, 2>(cfg, a, b, s, launches);
   }
-  if (v == 0) return launch_waves_t<2, 0>(cfg, a, b, s, launches);
-  if (v == 1) return launch_waves_t<2, 1>(cfg, a, b, s, launches);
-  return launch_waves_t<2, 2>(cfg, a, b, s, launches);
+  if (v == 0) return launch_waves_v<2, 0>(cfg, a, b, s, launches);
+  if (v == 1) return launch_waves_v<2, 1>(cfg, a, b, s, launches);
+  return launch_waves_v<2, 2>(cfg, a, b, s, launches);
 }
 
 template <int LPL, int V>

@@ -53,9 +53,10 @@ struct PixLM {
 static_assert(sizeof(PixLM) == 576, "PixLM is one 576-byte record");
 
 // Per wave: the trial kernel's cursor, the pixels it passes to the next wave
-// and to the accept kernel, and the accept kernel's cursor.
+// (those whose next step has to be solved and those that hold it already),
+// and the pixels it passes to the accept kernel.
 struct WaveCounters {
-  unsigned int cur_trial, n_next, n_acc, cur_acc;
+  unsigned int cur_trial, n_solve, n_reuse, n_acc;
 };
 
 // Floats of one pixel's staged trial (accepted trial -> accept kernel): 23
@@ -69,10 +70,12 @@ __host__ __device__ constexpr int stage_floats() { return stage_floats_for(LPL);
 struct WaveArgs {
   PixLM* state;                // [chunk]
   float* stage;                // [chunk][stage_floats]
-  uint32_t* act0;              // pixels iterating in even / odd waves
-  uint32_t* act1;
+  uint32_t* act0;              // pixels iterating in even / odd waves: those to solve from
+  uint32_t* act1;              // the front, those that reuse a step from the back
+  uint32_t cap;                // entries of each list
   uint32_t* accl;              // pixels accepted in the current wave
   WaveCounters* cnt;           // [waves], zeroed per chunk
+  uint32_t* cur_acc;           // the accept kernel's cursor, zeroed by each trial kernel
 };
 
 // Device memory of a wave-synchronous inversion, carved from one buffer.
