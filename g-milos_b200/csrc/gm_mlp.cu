@@ -13,8 +13,7 @@
 // Activations are written into the operand tile by the epilogue threads
 // themselves (the swizzle computed in place), so a tile's three layers run
 // back to back without leaving the SM.  Inference keeps two tiles in
-// flight per CTA, a producer warp issuing one tile's products while eight
-// epilogue warps work on the other's accumulator.
+// flight per CTA, each with eight epilogue warps, and a producer warp.
 //
 // Training runs per batch: (1) one fused kernel per 128-pixel tile for the
 // forward pass, the loss, and the backward pass through the activations
@@ -42,10 +41,10 @@ namespace gm {
 namespace mlp {
 namespace {
 
-// Inference and training kernels: 8 epilogue warps, two per tensor-memory
-// lane quarter -- warp w reads rows 32 (w % 4) .. + 31 of the accumulator,
-// and the two warpgroups split each epilogue's columns (and the input
-// features) in halves; inference adds a producer warp.  The weight-gradient
+// Inference and training kernels: 8 epilogue warps a tile, two per
+// tensor-memory lane quarter -- warp w reads rows 32 (w % 4) .. + 31 of the
+// accumulator, and the two warpgroups split each epilogue's columns in
+// halves; inference has two tiles' worth and a producer warp.  The weight-gradient
 // kernel: 4 warps, one row each.
 constexpr int kThreads = 256;
 constexpr int kWThreads = 128;
@@ -274,7 +273,7 @@ struct Job {
   uint16_t rows, tcol;
   uint8_t acc, end;
 };
-constexpr int kInferJobs = 4, kTrainJobs = 7;
+constexpr int kTrainJobs = 7;
 __constant__ Job c_jobs[kTrainJobs] = {
     {kMapW1, 2, 0, 0, 256, 0, 0, 1},      // Z1 = X W1^T
     {kMapW2, 2, 0, 0, 256, 256, 0, 0},    // Z2 = H1 W2^T (K 0..127); column 0 in inference
@@ -366,40 +365,53 @@ __device__ bool run_job(const Job& j, const Job* next, bool train, const NetMaps
   return true;
 }
 
-// Load a tile's inputs (batch rows row0.., pixel idx[row] or the row itself)
-// standardised and rounded to BF16 into the activation atoms 0-1; this
-// thread's row r, features [64 half, 64 half + 64) (atom `half`).  Rows of
-// 4 nl floats start on 16-byte boundaries and the feature count is a
-// multiple of 4, so every 4-feature group is read whole or not at all.
+// Load a tile's inputs (batch rows row0..,  pixel idx[row] or the row itself)
+// standardised and rounded to BF16 into the activation atoms 0-1.  Warp w of
+// the NW that share the work takes the rows 128 / NW w .., a row at a time:
+// lane f holds features 4 f .. 4 f + 3, so a row is one coalesced read (a row
+// per lane instead touched 32 lines an instruction and took 10 k cycles a
+// tile) and the lane's standardisation stays in registers.  Rows of 4 nl
+// floats start on 16-byte boundaries and the feature count is a multiple of
+// 4, so every 4-feature group is read whole or not at all.
+template <int NW>
 __device__ __forceinline__ void load_x(const float* spar, const float* __restrict__ iquv,
                                        const uint32_t* __restrict__ idx, int64_t row0, int64_t n, int nl,
-                                       uint32_t sA, int r, int half) {
-  const int64_t b = row0 + r;
-  const int F = 4 * nl;
-  const float4* src = nullptr;
-  if (b < n) src = reinterpret_cast<const float4*>(iquv + (idx ? (int64_t)idx[b] : b) * F);
-  const float4* mean = reinterpret_cast<const float4*>(spar + 512);
-  const float4* scale = reinterpret_cast<const float4*>(spar + 640);
-#pragma unroll 2
-  for (int c = 8 * half; c < 8 * half + 8; ++c) {
-    float v[8];
+                                       uint32_t sA, int w) {
+  constexpr int R = kTile / NW, U = 8;   // rows of this warp, reads in flight
+  const int f = threadIdx.x & 31;
+  const float4 mu = reinterpret_cast<const float4*>(spar + 512)[f];
+  const float4 sc = reinterpret_cast<const float4*>(spar + 640)[f];
+  const uint32_t atom = sA + (uint32_t)(f >> 4) * 16384u;
+#pragma unroll 1
+  for (int r0 = w * R; r0 < w * R + R; r0 += U) {
+    float4 x[U];
 #pragma unroll
-    for (int g = 0; g < 2; ++g) {
-      const int f4 = 2 * c + g;   // 4-feature group
-      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (src && 4 * f4 < F) {
-        const float4 xi = __ldg(src + f4), mu = mean[f4], sc = scale[f4];
-        x = make_float4((xi.x - mu.x) * sc.x, (xi.y - mu.y) * sc.y, (xi.z - mu.z) * sc.z, (xi.w - mu.w) * sc.w);
-      }
-      v[4 * g] = x.x;
-      v[4 * g + 1] = x.y;
-      v[4 * g + 2] = x.z;
-      v[4 * g + 3] = x.w;
+    for (int u = 0; u < U; ++u) {
+      const int64_t b = row0 + r0 + u;
+      if (b < n && f < nl)
+        x[u] = __ldg(reinterpret_cast<const float4*>(iquv + (idx ? (int64_t)idx[b] : b) * (4 * nl)) + f);
     }
-    const uint32_t w[4] = {pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]),
-                           pack_bf16(v[6], v[7])};
-    st_chunk(sA + (c >> 3) * 16384u, r, c & 7, w);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int r = r0 + u;
+      uint32_t lo = 0u, hi = 0u;
+      if (row0 + r < n && f < nl) {
+        lo = pack_bf16((x[u].x - mu.x) * sc.x, (x[u].y - mu.y) * sc.y);
+        hi = pack_bf16((x[u].z - mu.z) * sc.z, (x[u].w - mu.w) * sc.w);
+      }
+      const uint32_t a = atom + (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((((f >> 1) & 7) ^ (r & 7)) << 4) +
+                                           8 * (f & 1));
+      asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a), "r"(lo), "r"(hi) : "memory");
+    }
   }
+}
+
+// Ask for the lines of a tile's inputs in L2 (thread i of the 256 that share it).
+__device__ __forceinline__ void prefetch_x(const float* __restrict__ iquv, int64_t row0, int64_t n, int nl, int i) {
+  const int64_t rows = n - row0 < kTile ? n - row0 : kTile;
+  const char* p = reinterpret_cast<const char*>(iquv + row0 * (4 * nl));
+  for (int64_t o = 128 * (int64_t)i; o < rows * (16 * nl); o += 128 * 256)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p + o));
 }
 
 // Epilogue of a hidden layer over the accumulator at tensor column zcol:
@@ -552,18 +564,27 @@ __device__ __forceinline__ void teardown(Bars* B, Pipe& p, uint32_t ncols, int* 
 
 // ---------------------------------------------------------------- inference
 // Persistent and warp-specialised, two 128-pixel tiles in flight per CTA
-// (slots 0 and 1: each its own activation tile in shared memory and 256
-// tensor-memory columns).  Warps 0-7 are epilogue warps: they load a
-// slot's inputs, and after each of its products turn the accumulator into
-// the next operand (GELU) or the start models; warp 8's first thread
-// streams the weights through two 32 KB stages by TMA and issues the
-// products.  While the epilogue warps work on one slot, the tensor core
-// works on the other: per pair of tiles (A in slot 0, B in slot 1) the
-// products run L0(A) L0(B) L1(A) L1(B) L2(A) L2(B) and the epilogues
-// E0(A) E0(B) E1(A) E1(B) OUT(A) X(A') OUT(B) X(B'), each product waiting
-// for the epilogue that wrote its operand (hready, all 256 epilogue
-// threads arrive) and each epilogue for its product (zready, a commit).
-constexpr int kIThreads = 288;                 // 8 epilogue warps + the producer warp
+// (slots 0 and 1: each its own activation tile in shared memory, 256
+// tensor-memory columns and eight epilogue warps).  Warps 8 s .. 8 s + 7 load
+// slot s's inputs, and after each of its products turn the accumulator into
+// the next operand (GELU) or the start models; warp 16's first thread streams
+// the weights through two 32 KB stages by TMA and issues the products.  Per
+// pair of tiles (A in slot 0, B in slot 1) the products run L0(A) L0(B) L1(A)
+// L1(B) L2(A) L2(B); each waits for the epilogue that wrote its operand
+// (hready, the slot's 256 threads arrive) and each epilogue for its product
+// (zready, a commit), so the slots' epilogues overlap each other and the
+// products of the other slot.
+//
+// Bound by the epilogues: 512 GELUs a pixel, two special-function operations
+// each, 60 us of that unit for 2^18 pixels, and about as many issue slots.
+// Eight warps serving both slots in turn, each thread reading a row of inputs
+// (10 k of a tile's 42 k cycles), took 197 us; sixteen, each pair of
+// warpgroups on its own slot, rows read coalesced from lines asked for a
+// tile ahead, and one warpgroup loading the next tile while the other forms
+// the start models: 163 us (that unit 43 % active; a slot still waits 9 k of
+// 36 k cycles for its products).
+constexpr int kIEpi = 256;                     // epilogue threads of a slot
+constexpr int kIThreads = 2 * kIEpi + 32;      // and the producer warp
 constexpr uint32_t kIAct = 65536;              // one slot's activation tile (4 K-atoms)
 constexpr uint32_t kIW = 2 * kIAct;            // weight stages
 constexpr uint32_t kIStage = 32768;            // one K-atom of a 256-row weight
@@ -670,7 +691,7 @@ mlp_infer_kernel(const __grid_constant__ NetMaps nm, const InferArgs a) {
   __syncthreads();
   tc_fence_after();
   const uint32_t wbase = base + kIW;
-  if (warp == 8) {
+  if (warp == 2 * kIEpi / 32) {
     // ---- producer: weights and products
     Prod P;
     bool ok = true;
@@ -731,54 +752,47 @@ mlp_infer_kernel(const __grid_constant__ NetMaps nm, const InferArgs a) {
       mbar_wait(&B->fin, 0, &B->abort, a.err, kErrWaitMma, false);
     }
   } else {
-    // ---- epilogue warps
-    const int row = tid & (kTile - 1), half = tid >> 7;   // accumulator row, column half
-    const uint32_t qoff = (uint32_t)((warp & 3) * 32) << 16;
-    uint32_t zph[2] = {0, 0};
+    // ---- epilogue warps of slot sl: accumulator row, column half
+    const int sl = tid / kIEpi, row = tid & (kTile - 1), half = (tid / kTile) & 1;
+    const uint32_t trow = B->tmem + 256u * sl + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t act = base + sl * kIAct;
+    uint32_t zph = 0;
     bool ok = true;
-    auto zwait = [&](int sl) {
-      ok = ok && mbar_wait(&B->zready[sl], zph[sl], &B->abort, a.err, kErrWaitMma);
-      zph[sl] ^= 1u;
+    auto zwait = [&] {
+      ok = mbar_wait(&B->zready[sl], zph, &B->abort, a.err, kErrWaitMma);
+      zph ^= 1u;
       tc_fence_after();
       return ok;
     };
-    for (int sl = 0; sl < 2; ++sl) {
-      const int64_t t = blockIdx.x + sl * G;
-      if (t < tiles) {
-        load_x(spar, a.iquv, nullptr, t * kTile, a.n, a.nl, base + sl * kIAct, row, half);
+    int64_t t = blockIdx.x + sl * G;
+    if (t < tiles) {
+      load_x<8>(spar, a.iquv, nullptr, t * kTile, a.n, a.nl, act, warp & 7);
+      epi_arrive(&B->hready[sl]);
+    }
+    for (; t < tiles && ok; t += 2 * G) {
+      const int64_t tn = t + 2 * G;   // this slot's next tile
+      if (tn < tiles) prefetch_x(a.iquv, tn * kTile, a.n, a.nl, tid & (kIEpi - 1));
+#pragma unroll 1
+      for (int L = 0; L < 2; ++L) {
+        if (!zwait()) break;
+        hidden_epilogue(trow, 0, spar + 256 * L, act, row, half, nullptr);
         epi_arrive(&B->hready[sl]);
       }
-    }
-    for (int64_t tA = blockIdx.x; tA < tiles && ok; tA += 2 * G) {
-      const int nslot = tA + G < tiles ? 2 : 1;
-      for (int L = 0; L < 2 && ok; ++L)
-        for (int sl = 0; sl < nslot; ++sl) {
-          if (!zwait(sl)) break;
-          hidden_epilogue(B->tmem + 256u * sl + qoff, 0, spar + 256 * L, base + sl * kIAct, row, half, nullptr);
-          epi_arrive(&B->hready[sl]);
-        }
-      for (int sl = 0; sl < nslot && ok; ++sl) {
-        if (!zwait(sl)) break;
-        const int64_t t = tA + sl * G;
-        if (half == 0) {
-          const int64_t b = t * kTile + row;
-          float o[16];
-          tmem_ld16(B->tmem + 256u * sl + qoff, o);
-          if (b < a.n) {
-            float y[kOut];
+      if (!ok || !zwait()) break;
+      // one warpgroup reads the outputs while the other loads the next tile
+      float o[16];
+      if (half == 0) tmem_ld16(trow, o);
+      else if (tn < tiles) load_x<4>(spar, a.iquv, nullptr, tn * kTile, a.n, a.nl, act, warp & 3);
+      if (tn < tiles) epi_arrive(&B->hready[sl]);
+      const int64_t b = t * kTile + row;
+      if (half == 0 && b < a.n) {
+        float y[kOut];
 #pragma unroll
-            for (int j = 0; j < kOut; ++j) y[j] = (o[j] + a.p->b3[j]) * a.p->out_scale[j] + a.p->out_mean[j];
-            double m[11];
-            outputs_to_model(y, a.guess, a.fix, m);
+        for (int j = 0; j < kOut; ++j) y[j] = (o[j] + a.p->b3[j]) * a.p->out_scale[j] + a.p->out_mean[j];
+        double m[11];
+        outputs_to_model(y, a.guess, a.fix, m);
 #pragma unroll
-            for (int i = 0; i < 11; ++i) a.models[b * 11 + i] = m[i];
-          }
-        }
-        // this slot's next tile
-        if (t + 2 * G < tiles) {
-          load_x(spar, a.iquv, nullptr, (t + 2 * G) * kTile, a.n, a.nl, base + sl * kIAct, row, half);
-          epi_arrive(&B->hready[sl]);
-        }
+        for (int i = 0; i < 11; ++i) a.models[b * 11 + i] = m[i];
       }
     }
   }
@@ -817,7 +831,7 @@ mlp_train_kernel(const __grid_constant__ NetMaps nm, const __grid_constant__ Act
     // the previous tile's stores must have read the operand tiles
     if (tid == 0) tma_store_wait_read();
     __syncthreads();
-    load_x(spar, a.iquv, a.idx, t * kTile, a.n, a.nl, sA, row, half);
+    load_x<8>(spar, a.iquv, a.idx, t * kTile, a.n, a.nl, sA, warp);
     fence_proxy_async();
     __syncthreads();
     if (tid == 0) {
