@@ -41,12 +41,12 @@ namespace gm {
 namespace mlp {
 namespace {
 
-// Inference and training kernels: 8 epilogue warps a tile, two per
-// tensor-memory lane quarter -- warp w reads rows 32 (w % 4) .. + 31 of the
-// accumulator, and the two warpgroups split each epilogue's columns in
-// halves; inference has two tiles' worth and a producer warp.  The weight-gradient
+// Inference kernel: 8 epilogue warps a tile, two tiles' worth, and a producer
+// warp; training kernel: 16 epilogue warps.  Warp w reads rows
+// 32 (w % 4) .. + 31 of the accumulator, and a tile's warpgroups split each
+// epilogue's columns in equal parts.  The weight-gradient
 // kernel: 4 warps, one row each.
-constexpr int kThreads = 256;
+constexpr int kThreads = 512;
 constexpr int kWThreads = 128;
 constexpr uint64_t kWaitNs = 2000000000ull;   // a wait gives up after 2 s
 
@@ -276,7 +276,7 @@ struct Job {
 constexpr int kTrainJobs = 7;
 __constant__ Job c_jobs[kTrainJobs] = {
     {kMapW1, 2, 0, 0, 256, 0, 0, 1},      // Z1 = X W1^T
-    {kMapW2, 2, 0, 0, 256, 256, 0, 0},    // Z2 = H1 W2^T (K 0..127); column 0 in inference
+    {kMapW2, 2, 0, 0, 256, 256, 0, 0},    // Z2 = H1 W2^T (K 0..127)
     {kMapW2, 2, 2, 0, 256, 256, 1, 1},    //            (K 128..255)
     {kMapW3, 4, 0, 0, 16, 0, 0, 1},       // out = H2 W3^T
     {kMapW3t, 1, 0, 1, 256, 0, 0, 1},     // dH2 = dOut W3
@@ -284,15 +284,11 @@ __constant__ Job c_jobs[kTrainJobs] = {
     {kMapW2t, 2, 2, 0, 256, 256, 1, 1},   //            (K 128..255)
 };
 // weight blocks of layer L: [first, last)
-__device__ __forceinline__ int layer_first(int L, bool train) {
-  return L == 0 ? 0 : (L == 1 ? 1 : (train ? L + 1 : 3));
-}
-__device__ __forceinline__ int layer_last(int L, bool train) {
-  return L == 0 ? 1 : (L == 1 ? 3 : (L == 4 ? 7 : (train ? L + 2 : 4)));
-}
+__device__ __forceinline__ int layer_first(int L) { return L == 0 ? 0 : (L == 1 ? 1 : L + 1); }
+__device__ __forceinline__ int layer_last(int L) { return L == 0 ? 1 : (L == 1 ? 3 : (L == 4 ? 7 : L + 2)); }
 
 struct Bars {
-  uint64_t full[2], empty[2], mma;
+  uint64_t full[2], mma;
   uint32_t tmem;
   int abort;
 };
@@ -320,48 +316,37 @@ __device__ __forceinline__ void mma_job(const Job& j, uint32_t tmem, uint32_t tc
 }
 
 // Producer / issuer state (thread 0), and the epilogue barrier's parity
-// (all threads).
+// (all threads).  Weight blocks run in the order of c_jobs, tile after tile,
+// through the two stages in turn.
 struct Pipe {
-  uint32_t fph[2] = {0, 0}, eph[2] = {0, 0};   // next parity to wait for
-  bool pend[2] = {false, false};                // a commit on empty[s] not yet waited for
+  uint32_t fph[2] = {0, 0};                     // next parity to wait for
   bool inflight[2] = {false, false};            // a load into stage s not yet waited for
   uint32_t mph = 0;
-  int g = 0;                                    // weight blocks issued so far
+  int64_t g = 0, loaded = 0;                    // weight blocks run and loads started so far
 };
 
-__device__ __forceinline__ void start_load(const Job& j, const NetMaps& nm, Bars* B, uint32_t base, int s,
-                                           Pipe& p) {
-  load_job(j, nm, base + kSW + s * kStage, &B->full[s]);
-  p.inflight[s] = true;
+// Thread 0, with the products of every block run so far complete: start the
+// loads of the next two blocks of `total` that are not on their way yet.
+__device__ __forceinline__ void load_ahead(int64_t total, const NetMaps& nm, Bars* B, uint32_t base, Pipe& p) {
+  while (p.loaded < total && p.loaded < p.g + 2) {
+    const int s = (int)(p.loaded & 1);
+    load_job(c_jobs[p.loaded % kTrainJobs], nm, base + kSW + s * kStage, &B->full[s]);
+    p.inflight[s] = true;
+    ++p.loaded;
+  }
 }
 
-// Thread 0: run weight block `j`: wait for its weights, issue its products,
-// signal the stage free and (layer end) the epilogue, then start loading
-// `next` into the other stage once the products that last read it are done.
-// Returns false on abort.
-__device__ bool run_job(const Job& j, const Job* next, bool train, const NetMaps& nm, Bars* B, uint32_t base,
-                        Pipe& p, int* err) {
-  const int s = p.g & 1;
-  const uint32_t stage = base + kSW + s * kStage;
+// Thread 0: run the next weight block: wait for its weights, issue its
+// products, signal the epilogue at the end of a layer.  Returns false on abort.
+__device__ bool run_job(const Job& j, Bars* B, uint32_t base, Pipe& p, int* err) {
+  const int s = (int)(p.g & 1);
   if (!mbar_wait(&B->full[s], p.fph[s], &B->abort, err, kErrWaitLoad)) return false;
   p.fph[s] ^= 1u;
   p.inflight[s] = false;
   tc_fence_after();
-  const uint32_t tcol = (train || j.tcol < 256) ? j.tcol : 0u;
-  mma_job(j, B->tmem, tcol, base + kSA, base + kSD, stage);
-  mma_commit(&B->empty[s]);
-  p.pend[s] = true;
+  mma_job(j, B->tmem, j.tcol, base + kSA, base + kSD, base + kSW + s * kStage);
   if (j.end) mma_commit(&B->mma);
   ++p.g;
-  if (next) {
-    const int o = s ^ 1;
-    if (p.pend[o]) {
-      if (!mbar_wait(&B->empty[o], p.eph[o], &B->abort, err, kErrWaitStage)) return false;
-      p.eph[o] ^= 1u;
-      p.pend[o] = false;
-    }
-    start_load(*next, nm, B, base, o, p);
-  }
   return true;
 }
 
@@ -378,7 +363,9 @@ __device__ __forceinline__ void load_x(const float* spar, const float* __restric
                                        const uint32_t* __restrict__ idx, int64_t row0, int64_t n, int nl,
                                        uint32_t sA, int w) {
   constexpr int R = kTile / NW, U = 8;   // rows of this warp, reads in flight
+  static_assert(R % U == 0 && R <= 32, "a warp's rows");
   const int f = threadIdx.x & 31;
+  const uint32_t mine = idx && f < R && row0 + w * R + f < n ? __ldg(idx + row0 + w * R + f) : 0u;
   const float4 mu = reinterpret_cast<const float4*>(spar + 512)[f];
   const float4 sc = reinterpret_cast<const float4*>(spar + 640)[f];
   const uint32_t atom = sA + (uint32_t)(f >> 4) * 16384u;
@@ -388,8 +375,9 @@ __device__ __forceinline__ void load_x(const float* spar, const float* __restric
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int64_t b = row0 + r0 + u;
+      const int64_t p = idx ? (int64_t)__shfl_sync(0xffffffffu, mine, r0 + u - w * R) : b;
       if (b < n && f < nl)
-        x[u] = __ldg(reinterpret_cast<const float4*>(iquv + (idx ? (int64_t)idx[b] : b) * (4 * nl)) + f);
+        x[u] = __ldg(reinterpret_cast<const float4*>(iquv + p * (4 * nl)) + f);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -416,12 +404,12 @@ __device__ __forceinline__ void prefetch_x(const float* __restrict__ iquv, int64
 
 // Epilogue of a hidden layer over the accumulator at tensor column zcol:
 // h = GELU(z + bias) into the activation atoms (K = feature); with zspill,
-// z + bias also to zspill[0..256) (this row).  This thread: row r, columns
-// [128 half, 128 half + 128) (atoms 2 half, 2 half + 1), 32 at a time, the
-// next 32 columns' tensor-memory load in flight while these are processed.
-// bias: 256 floats in shared memory.
+// z + bias also to zspill[128 c] (columns 4 c .. 4 c + 3 of this row: a warp's
+// rows are neighbours there).  This thread: row r, part `part` of PARTS of
+// the 256 columns, 32 at a time, the next 32 columns' tensor-memory load in
+// flight while these are processed.  bias: 256 floats in shared memory.
 __device__ __forceinline__ void hidden_chunk(const uint32_t (&zr)[32], int q, const float* bias, uint32_t sA,
-                                             int r, float* zspill) {
+                                             int r, float4* zspill) {
   float z[32];
   const float4* b4 = reinterpret_cast<const float4*>(bias + 32 * q);
 #pragma unroll
@@ -433,9 +421,9 @@ __device__ __forceinline__ void hidden_chunk(const uint32_t (&zr)[32], int q, co
     z[4 * u + 3] = __uint_as_float(zr[4 * u + 3]) + bv.w;
   }
   if (zspill) {
-    float4* dst = reinterpret_cast<float4*>(zspill + 32 * q);
 #pragma unroll
-    for (int u = 0; u < 8; ++u) dst[u] = make_float4(z[4 * u], z[4 * u + 1], z[4 * u + 2], z[4 * u + 3]);
+    for (int u = 0; u < 8; ++u)
+      zspill[(8 * q + u) * kTile] = make_float4(z[4 * u], z[4 * u + 1], z[4 * u + 2], z[4 * u + 3]);
   }
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
@@ -446,19 +434,21 @@ __device__ __forceinline__ void hidden_chunk(const uint32_t (&zr)[32], int q, co
   }
 }
 
+template <int PARTS>
 __device__ __forceinline__ void hidden_epilogue(uint32_t tmem_row, uint32_t zcol, const float* bias, uint32_t sA,
-                                                int r, int half, float* zspill) {
-  const int q0 = 4 * half;
+                                                int r, int part, float4* zspill) {
+  constexpr int N = 8 / PARTS;   // chunks of 32 columns
+  const int q0 = N * part;
   const uint32_t t0 = tmem_row + zcol + 32 * q0;
   uint32_t za[32], zb[32];
   tmem_issue32(t0, za);
 #pragma unroll
-  for (int j = 0; j < 4; j += 2) {
+  for (int j = 0; j < N; j += 2) {
     tmem_wait32(za);
     tmem_issue32(t0 + 32 * (j + 1), zb);
     hidden_chunk(za, q0 + j, bias, sA, r, zspill);
     tmem_wait32(zb);
-    if (j + 2 < 4) tmem_issue32(t0 + 32 * (j + 2), za);
+    if (j + 2 < N) tmem_issue32(t0 + 32 * (j + 2), za);
     hidden_chunk(zb, q0 + j + 1, bias, sA, r, zspill);
   }
 }
@@ -516,7 +506,7 @@ struct TrainKArgs {
   int64_t n;               // rows of this batch (a multiple of 128)
   int nl;
   float gscale;            // d loss / d output per unit of error: 2 / (rows x 9)
-  float* zspill;           // [rows][256] pre-activations of layer 1
+  float* zspill;           // [tiles][64][128][4] pre-activations of layer 1 (4-column group, row)
   float* loss;             // sum of squared errors (atomic)
   int* err;
 };
@@ -531,8 +521,6 @@ __device__ __forceinline__ void setup(Bars* B, uint32_t ncols) {
   if (tid == 0) {
     mbar_init(&B->full[0], 1);
     mbar_init(&B->full[1], 1);
-    mbar_init(&B->empty[0], 1);
-    mbar_init(&B->empty[1], 1);
     mbar_init(&B->mma, 1);
     B->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -775,7 +763,7 @@ mlp_infer_kernel(const __grid_constant__ NetMaps nm, const InferArgs a) {
 #pragma unroll 1
       for (int L = 0; L < 2; ++L) {
         if (!zwait()) break;
-        hidden_epilogue(trow, 0, spar + 256 * L, act, row, half, nullptr);
+        hidden_epilogue<2>(trow, 0, spar + 256 * L, act, row, half, nullptr);
         epi_arrive(&B->hready[sl]);
       }
       if (!ok || !zwait()) break;
@@ -808,13 +796,21 @@ mlp_infer_kernel(const __grid_constant__ NetMaps nm, const InferArgs a) {
 // zspill), Z2 256..511 (kept until dZ2), out 0..15, dH2 0..255, dH1
 // 256..511.  X, H1, H2, dOut, dZ2, dZ1 go row-major to global memory (TMA
 // stores of the operand tiles) for the weight gradients.
+//
+// Bound by one tile's chain of phases (a batch of 8192 has 64 tiles on 148
+// SMs), so each is cut: 16 warps share the epilogues, the next two weight
+// blocks load while an epilogue runs, Z1's spill is laid out by column group so
+// that a warp's rows are neighbours, and a warp reads its rows of X in one
+// batch.  65 -> 43.5 us for 8192 rows (8 warps; the spill a row per thread,
+// 14 k of 96 k cycles each way; the second half of W2 loaded after the first
+// half's products; X in two batches behind their indices, 19 k cycles).
 __global__ void __launch_bounds__(kThreads, 1)
 mlp_train_kernel(const __grid_constant__ NetMaps nm, const __grid_constant__ ActMaps am, const TrainKArgs a) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t base = (saddr(smem_raw) + 1023u) & ~1023u;
   Bars* B = reinterpret_cast<Bars*>(smem_raw + (base - saddr(smem_raw)) + kSBar);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int row = tid & (kTile - 1), half = tid >> 7;   // accumulator row, column half
+  const int row = tid & (kTile - 1), part = tid / kTile;   // accumulator row, column quarter
   float* spar = reinterpret_cast<float*>(smem_raw + (base - saddr(smem_raw)) + kSPar);
   stage_params(a.p, spar);
   setup(B, 512);
@@ -823,15 +819,16 @@ mlp_train_kernel(const __grid_constant__ NetMaps nm, const __grid_constant__ Act
   const int64_t tiles = a.n / kTile;
   Pipe p;
   bool ok = true;
-  if (tid == 0 && (int64_t)blockIdx.x < tiles) start_load(c_jobs[0], nm, B, base, 0, p);
+  // weight blocks of this CTA's tiles
+  const int64_t blocks = (int64_t)blockIdx.x < tiles ? (tiles - 1 - blockIdx.x) / gridDim.x * kTrainJobs + kTrainJobs : 0;
+  if (tid == 0) load_ahead(blocks, nm, B, base, p);
   for (int64_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-    const bool last_tile = t + gridDim.x >= tiles;
     const int64_t b = t * kTile + row;   // this thread's batch row
-    float* zrow = a.zspill + b * kHid;
+    float4* zrow = reinterpret_cast<float4*>(a.zspill) + t * (kTile * kHid / 4) + row;
     // the previous tile's stores must have read the operand tiles
     if (tid == 0) tma_store_wait_read();
     __syncthreads();
-    load_x<8>(spar, a.iquv, a.idx, t * kTile, a.n, a.nl, sA, warp);
+    load_x<16>(spar, a.iquv, a.idx, t * kTile, a.n, a.nl, sA, warp);
     fence_proxy_async();
     __syncthreads();
     if (tid == 0) {
@@ -842,25 +839,24 @@ mlp_train_kernel(const __grid_constant__ NetMaps nm, const __grid_constant__ Act
     // five layers: 0 Z1, 1 Z2, 2 out, 3 dH2, 4 dH1
     for (int L = 0; L < 5 && ok; ++L) {
       if (tid == 0) {
-        for (int j = layer_first(L, true); j < layer_last(L, true) && ok; ++j) {
-          const Job* nx = (j + 1 < kTrainJobs) ? &c_jobs[j + 1] : (last_tile ? nullptr : &c_jobs[0]);
-          ok = run_job(c_jobs[j], nx, true, nm, B, base, p, a.err);
-        }
+        for (int j = layer_first(L); j < layer_last(L) && ok; ++j) ok = run_job(c_jobs[j], B, base, p, a.err);
       }
       ok = mbar_wait(&B->mma, p.mph, &B->abort, a.err, kErrWaitMma) && ok;
       p.mph ^= 1u;
+      // both stages' products are done: the next loads run beside the epilogue;
       // an epilogue that overwrites the activation tile waits for its stores
+      if (tid == 0 && ok) load_ahead(blocks, nm, B, base, p);
       if (tid == 0 && L != 2) tma_store_wait_read();
       __syncthreads();
       ok = ok && !B->abort;
       if (!ok) break;
       tc_fence_after();
       if (L == 0) {
-        hidden_epilogue(trow, 0, spar, sA, row, half, zrow);
+        hidden_epilogue<4>(trow, 0, spar, sA, row, part, zrow);
       } else if (L == 1) {
-        hidden_epilogue(trow, 256, spar + 256, sA, row, half, nullptr);
+        hidden_epilogue<4>(trow, 256, spar + 256, sA, row, part, nullptr);
       } else if (L == 2) {
-        if (half == 0) {   // the 9 outputs: the first warpgroup
+        if (part == 0) {   // the 9 outputs: the first warpgroup
           float o[16];
           tmem_ld16(trow, o);
           const float* yt = a.y16 + (int64_t)a.idx[b] * 16;
@@ -888,9 +884,9 @@ mlp_train_kernel(const __grid_constant__ NetMaps nm, const __grid_constant__ Act
       } else {
         // dZ = dH GELU'(Z): L 3 -> dZ2 (dH2 at column 0, Z2 at 256);
         // L 4 -> dZ1 (dH1 at column 256, Z1 from the spill); this
-        // warpgroup's half of the columns
+        // warpgroup's quarter of the columns
 #pragma unroll 1
-        for (int q = 4 * half; q < 4 * half + 4; ++q) {
+        for (int q = 2 * part; q < 2 * part + 2; ++q) {
           float dh[32], z[32];
           if (L == 3) {
             tmem_ld32(trow + 32 * q, dh);
@@ -899,10 +895,9 @@ mlp_train_kernel(const __grid_constant__ NetMaps nm, const __grid_constant__ Act
             for (int e = 0; e < 32; ++e) z[e] += spar[256 + 32 * q + e];
           } else {
             tmem_ld32(trow + 256 + 32 * q, dh);
-            const float4* src = reinterpret_cast<const float4*>(zrow + 32 * q);
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-              const float4 v = src[u];
+              const float4 v = zrow[(8 * q + u) * kTile];
               z[4 * u] = v.x;
               z[4 * u + 1] = v.y;
               z[4 * u + 2] = v.z;
