@@ -934,19 +934,30 @@ mlp_train_kernel(const __grid_constant__ NetMaps nm, const __grid_constant__ Act
   teardown(B, p, 512, a.err);
 }
 
-// ---------------------------------------------------------------- training: weight gradients
-// dW[m][n] += sum over a slice of the batch of A[b][m] Bm[b][n] for one
-// 128 x 64 block; both operands row-major in global memory, MN-major in the
-// product (8-row K groups 1024 bytes apart, 64-element M blocks 8 KB apart),
-// 4-stage TMA ring.  Products: 0 dW1 = G1^T X (4 blocks), 1 dW2 = G2^T H1
-// (8 blocks), 2 dW3^T = H2^T dOut (2 blocks, added transposed).  Blocks of
-// one product add their slices into the FP32 gradient.
+// ---------------------------------------------------------------- training: weight and bias gradients
+// The FP32 parameters of a gm_mlp in one flat index: w1, b1, w2, b2, w3, b3.
+constexpr int kNW1 = kHid * kIn, kNW2 = kHid * kHid, kNW3 = kOut * kHid;
+constexpr int kParams = kNW1 + kHid + kNW2 + kHid + kNW3 + kOut;
+constexpr int kOffB1 = kNW1, kOffW2 = kOffB1 + kHid, kOffB2 = kOffW2 + kNW2, kOffW3 = kOffB2 + kHid,
+              kOffB3 = kOffW3 + kNW3;
+constexpr int kPartStride = (kParams + 31) & ~31;   // a partial gradient; 16-byte stores into each
+static_assert(kOffW2 % 4 == 0 && kPartStride % 4 == 0, "aligned blocks of the weights");
+
+// One launch.  dW[m][n] = sum over a slice of the batch of A[b][m] Bm[b][n]
+// for one 128 x 64 block; both operands row-major in global memory, MN-major
+// in the product (8-row K groups 1024 bytes apart, 64-element M blocks 8 KB
+// apart), 4-stage TMA ring.  Products: 0 dW1 = G1^T X (4 blocks), 1 dW2 =
+// G2^T H1 (8 blocks), 2 dW3^T = H2^T dOut (2 blocks, stored transposed).  A
+// slice's blocks fill one partial gradient, which the optimiser sums in
+// order: the same gradient every time, where atomic additions into one
+// differed from run to run.  Two warps of one block per M range add up the
+// columns of its gradient operand as the stages pass, the bias gradients: a
+// kernel of its own read the gradients again and took as long as this one
+// (14.7 us a batch of 8192 rows).
 struct WgradArgs {
-  float* dw1;   // [256][128]
-  float* dw2;   // [256][256]
-  float* dw3;   // [9][256]
-  int64_t rows; // batch rows (a multiple of 64)
-  int kslices;  // batch slices per block
+  float* part;          // [kslices][kPartStride]
+  int64_t rows;         // batch rows (a multiple of 64)
+  int kslices;          // batch slices per block
   int* err;
 };
 struct WgradMaps {
@@ -979,10 +990,12 @@ mlp_wgrad_kernel(const __grid_constant__ WgradMaps wm, const WgradArgs a) {
   } else {
     g = 2; mb = blk - 12; nb = 0;
   }
+  // whose column sums this block forms: its A operand (G1, G2) or B (dOut)
+  const bool bias = g < 2 ? nb == 0 : mb == 0;
   if (tid == 0) {
     for (int s = 0; s < kWStages; ++s) {
       mbar_init(&B->full[s], 1);
-      mbar_init(&B->empty[s], 1);
+      mbar_init(&B->empty[s], bias ? 3 : 1);   // the products' commit and the two summing warps
     }
     mbar_init(&B->done, 1);
     B->abort = 0;
@@ -1042,6 +1055,33 @@ mlp_wgrad_kernel(const __grid_constant__ WgradMaps wm, const WgradArgs a) {
     }
     // the last commit covers every product issued (also after an abort)
     mma_commit(&B->done);
+  } else if (bias && (warp == 1 || warp == 2)) {
+    // two columns a thread, as 4 bytes of each swizzled 128-byte row
+    const int u = tid - 32;
+    const bool mine = g < 2 || u < kOut16 / 2;
+    const uint32_t col = (g < 2 ? (uint32_t)(u >> 5) * 8192u : 16384u) + 4u * (u & 3);
+    const uint32_t chunk = (uint32_t)(u & 31) >> 2;
+    float s0 = 0.f, s1 = 0.f;
+    for (int64_t k = k0; k < k1; ++k) {
+      const int s = (int)((k - k0) % kWStages);
+      if (!mbar_wait(&B->full[s], (uint32_t)((k - k0) / kWStages) & 1u, &B->abort, a.err, kErrWaitLoad)) break;
+      if (mine) {
+        const uint32_t st = base + s * kWStageBytes + col;
+#pragma unroll 16
+        for (uint32_t r = 0; r < 64; ++r) {
+          uint32_t v;
+          asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(st + r * 128u + ((chunk ^ (r & 7u)) << 4)));
+          s0 += __uint_as_float(v << 16);
+          s1 += __uint_as_float(v & 0xffff0000u);
+        }
+      }
+      __syncwarp();
+      if ((tid & 31) == 0) mbar_arrive(&B->empty[s]);
+    }
+    const int c = g == 0 ? kOffB1 + mb * 128 + 2 * u : (g == 1 ? kOffB2 + mb * 128 + 2 * u : kOffB3 + 2 * u);
+    float* part = a.part + (size_t)slice * kPartStride;
+    if (mine && c < kParams) part[c] = s0;
+    if (mine && c + 1 < kParams) part[c + 1] = s1;
   }
   __syncthreads();
   const bool ran = k1 > k0;
@@ -1056,19 +1096,15 @@ mlp_wgrad_kernel(const __grid_constant__ WgradMaps wm, const WgradArgs a) {
     for (int h = 0; h < 2; ++h) {
       float v[32];
       tmem_ld32(trow + 32 * h, v);
+      float* part = a.part + (size_t)slice * kPartStride;
       if (g < 2) {
         // this thread's 32 columns are contiguous in its row of dW1 / dW2
-        // (16-byte aligned): vector reductions, a quarter of the atomics
-        float* dst = (g == 0 ? a.dw1 + m * kIn : a.dw2 + m * kHid) + nb * 64 + 32 * h;
+        float4* dst = reinterpret_cast<float4*>(part + (g == 0 ? m * kIn : kOffW2 + m * kHid) + nb * 64 + 32 * h);
 #pragma unroll
-        for (int e = 0; e < 32; e += 4)
-          atomicAdd(reinterpret_cast<float4*>(dst + e), make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]));
-      } else {
-#pragma unroll 4
-        for (int e = 0; e < 32; ++e) {
-          const int n = nb * 64 + 32 * h + e;
-          if (n < kOut) atomicAdd(a.dw3 + n * kHid + m, v[e]);
-        }
+        for (int e = 0; e < 32; e += 4) dst[e / 4] = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+      } else if (h == 0) {
+#pragma unroll
+        for (int n = 0; n < kOut; ++n) part[kOffW3 + n * kHid + m] = v[n];
       }
     }
   }
@@ -1080,29 +1116,7 @@ mlp_wgrad_kernel(const __grid_constant__ WgradMaps wm, const WgradArgs a) {
   if (warp == 0) tmem_dealloc(B->tmem, 64);
 }
 
-// Bias gradients: column sums of the stored output gradients (BF16),
-// gridDim.x slices of the batch, blockIdx.y the layer.
-__global__ void mlp_bias_grad_kernel(const uint16_t* __restrict__ g1, const uint16_t* __restrict__ g2,
-                                     const uint16_t* __restrict__ g3, int64_t rows, float* db1, float* db2,
-                                     float* db3) {
-  const int which = blockIdx.y;
-  const int f = threadIdx.x;
-  const int width = which == 2 ? kG : kHid;
-  const int used = which == 2 ? kOut : kHid;
-  if (f >= used) return;
-  const uint16_t* g = which == 0 ? g1 : (which == 1 ? g2 : g3);
-  float* db = which == 0 ? db1 : (which == 1 ? db2 : db3);
-  const int64_t r0 = rows * blockIdx.x / gridDim.x, r1 = rows * (blockIdx.x + 1) / gridDim.x;
-  float s = 0.f;
-  for (int64_t r = r0; r < r1; ++r) s += __uint_as_float((uint32_t)g[r * width + f] << 16);
-  atomicAdd(db + f, s);
-}
-
 // ---------------------------------------------------------------- parameters
-// The FP32 parameters of a gm_mlp in one flat index: w1, b1, w2, b2, w3, b3.
-constexpr int kNW1 = kHid * kIn, kNW2 = kHid * kHid, kNW3 = kOut * kHid;
-constexpr int kParams = kNW1 + kHid + kNW2 + kHid + kNW3 + kOut;
-
 __device__ __forceinline__ float* param_at(gm_mlp* p, int i, bool* bias) {
   *bias = false;
   if (i < kNW1) return &p->w1[0][0] + i;
@@ -1147,24 +1161,38 @@ __global__ void mlp_pack_kernel(const gm_mlp* p, uint16_t* pack) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kParams; i += gridDim.x * blockDim.x) pack_one(p, pack, i);
 }
 
+// Gradient of flat parameter i: the sum of its partials in order.
+__device__ __forceinline__ float grad_at(const float* __restrict__ part, int slices, int i) {
+  float g = 0.f;
+#pragma unroll 8
+  for (int k = 0; k < slices; ++k) g += __ldg(part + (size_t)k * kPartStride + i);
+  return g;
+}
+
+// The gradient of a batch as a gm_mlp (checks).
+__global__ void mlp_grad_kernel(const float* part, int slices, gm_mlp* grad) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kParams; i += gridDim.x * blockDim.x) {
+    bool bias;
+    float* g = param_at(grad, i, &bias);
+    *g = grad_at(part, slices, i);
+  }
+}
+
 // Adam with decoupled weight decay (weights only) on every parameter, its
-// BF16 copy rewritten, its gradient cleared for the next batch.  c1, c2: the
-// bias corrections 1 / (1 - beta^t).
-__global__ void mlp_adam_kernel(gm_mlp* p, gm_mlp* grad, gm_mlp* m1, gm_mlp* m2, uint16_t* pack, float lr,
-                                float wd, float c1, float c2) {
+// BF16 copy rewritten.  c1, c2: the bias corrections 1 / (1 - beta^t).
+__global__ void mlp_adam_kernel(gm_mlp* p, const float* part, int slices, gm_mlp* m1, gm_mlp* m2,
+                                uint16_t* pack, float lr, float wd, float c1, float c2) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kParams; i += gridDim.x * blockDim.x) {
     bool bias;
     float* w = param_at(p, i, &bias);
-    float* g = param_at(grad, i, &bias);
     float* ma = param_at(m1, i, &bias);
     float* mb = param_at(m2, i, &bias);
-    const float gv = *g;
+    const float gv = grad_at(part, slices, i);
     const float av = 0.9f * *ma + 0.1f * gv;
     const float bv = 0.999f * *mb + 0.001f * gv * gv;
     *ma = av;
     *mb = bv;
     *w -= lr * ((av * c1) / (sqrtf(bv * c2) + 1e-8f) + (bias ? 0.f : wd * *w));
-    *g = 0.f;
     pack_one(p, pack, i);
   }
 }
@@ -1361,9 +1389,6 @@ int sm_count() {
   return n > 0 ? n : 1;
 }
 
-// A float array of a gm_mlp in device memory (no host dereference).
-float* field(gm_mlp* dev, size_t offset) { return reinterpret_cast<float*>(reinterpret_cast<char*>(dev) + offset); }
-
 // Device buffers of a training session, freed together.
 struct Buffers {
   std::vector<void*> owned;
@@ -1482,17 +1507,24 @@ cudaError_t train(gm_mlp* net, const TrainArgs& a, float* loss_out, gm_mlp* grad
   }
   gm_mlp *grad = nullptr, *m1 = nullptr, *m2 = nullptr;
   uint16_t *x = nullptr, *h1 = nullptr, *h2 = nullptr, *g1 = nullptr, *g2 = nullptr, *g3 = nullptr;
-  float *z = nullptr, *y16 = nullptr, *loss = nullptr;
+  float *z = nullptr, *y16 = nullptr, *loss = nullptr, *gpart = nullptr;
   uint32_t* idx = nullptr;
   double2* part = nullptr;
   const int64_t n = a.n;
+  const int sms = sm_count();
+  const int64_t tiles = B / kTile;
+  const int tgrid = (int)std::min<int64_t>(tiles, sms);
+  // one product block per SM; two (twice the slices) leave the products at
+  // 13.5 us and make the optimiser sum twice as many partials, 8.7 us for 6.6
+  const int kslices = (int)std::max<int64_t>(1, std::min<int64_t>(B / 64, sms / kWBlocks));
   if ((e = buf.get(&grad, 1)) != cudaSuccess || (e = buf.get(&m1, 1)) != cudaSuccess ||
       (e = buf.get(&m2, 1)) != cudaSuccess || (e = buf.get(&x, (size_t)B * kIn)) != cudaSuccess ||
       (e = buf.get(&h1, (size_t)B * kHid)) != cudaSuccess || (e = buf.get(&h2, (size_t)B * kHid)) != cudaSuccess ||
       (e = buf.get(&g1, (size_t)B * kHid)) != cudaSuccess || (e = buf.get(&g2, (size_t)B * kHid)) != cudaSuccess ||
       (e = buf.get(&g3, (size_t)B * kG)) != cudaSuccess || (e = buf.get(&z, (size_t)B * kHid)) != cudaSuccess ||
       (e = buf.get(&y16, (size_t)n * 16)) != cudaSuccess || (e = buf.get(&idx, (size_t)n)) != cudaSuccess ||
-      (e = buf.get(&loss, 1)) != cudaSuccess || (e = buf.get(&part, (size_t)kMomBlocks * kMom)) != cudaSuccess) {
+      (e = buf.get(&loss, 1)) != cudaSuccess || (e = buf.get(&part, (size_t)kMomBlocks * kMom)) != cudaSuccess ||
+      (e = buf.get(&gpart, (size_t)kslices * kPartStride)) != cudaSuccess) {
     devnet_destroy(&d);
     return fail("device allocation", e);
   }
@@ -1525,11 +1557,6 @@ cudaError_t train(gm_mlp* net, const TrainArgs& a, float* loss_out, gm_mlp* grad
     devnet_destroy(&d);
     return fail("kernel attributes", e);
   }
-  const int sms = sm_count();
-  const int64_t tiles = B / kTile;
-  const int tgrid = (int)std::min<int64_t>(tiles, sms);
-  const int kslices = (int)std::max<int64_t>(1, std::min<int64_t>(B / 64, sms / kWBlocks));
-  const int bias_blocks = (int)std::max<int64_t>(1, std::min<int64_t>(B / 256, 64));
   const int epochs = a.grads_only ? 1 : std::max(1, a.epochs);
   const int64_t steps_per_epoch = n / B;
   const int64_t total = steps_per_epoch * epochs;
@@ -1558,13 +1585,8 @@ cudaError_t train(gm_mlp* net, const TrainArgs& a, float* loss_out, gm_mlp* grad
       ka.loss = loss;
       ka.err = err;
       mlp_train_kernel<<<tgrid, kThreads, kSmemBytes, s>>>(nm, am, ka);
-      mlp_bias_grad_kernel<<<dim3(bias_blocks, 3), 256, 0, s>>>(g1, g2, g3, B, field(grad, offsetof(gm_mlp, b1)),
-                                                                field(grad, offsetof(gm_mlp, b2)),
-                                                                field(grad, offsetof(gm_mlp, b3)));
       WgradArgs wa{};
-      wa.dw1 = field(grad, offsetof(gm_mlp, w1));
-      wa.dw2 = field(grad, offsetof(gm_mlp, w2));
-      wa.dw3 = field(grad, offsetof(gm_mlp, w3));
+      wa.part = gpart;
       wa.rows = B;
       wa.kslices = kslices;
       wa.err = err;
@@ -1574,7 +1596,7 @@ cudaError_t train(gm_mlp* net, const TrainArgs& a, float* loss_out, gm_mlp* grad
         const double lr = a.lr * 0.5 * (1.0 + std::cos(M_PI * (double)step / (double)std::max<int64_t>(1, total)));
         const float c1 = (float)(1.0 / (1.0 - std::pow(0.9, (double)t_adam)));
         const float c2 = (float)(1.0 / (1.0 - std::pow(0.999, (double)t_adam)));
-        mlp_adam_kernel<<<(kParams + 255) / 256, 256, 0, s>>>(d.p, grad, m1, m2, d.pack, (float)lr,
+        mlp_adam_kernel<<<(kParams + 255) / 256, 256, 0, s>>>(d.p, gpart, kslices, m1, m2, d.pack, (float)lr,
                                                               a.weight_decay, c1, c2);
       }
       e = cudaGetLastError();
@@ -1593,7 +1615,11 @@ cudaError_t train(gm_mlp* net, const TrainArgs& a, float* loss_out, gm_mlp* grad
   if (e == cudaSuccess) {
     const int64_t steps0 = net->steps;
     if (a.grads_only) {
-      if (grads_out) e = cudaMemcpy(grads_out, grad, sizeof(gm_mlp), cudaMemcpyDeviceToHost);
+      if (grads_out) {
+        mlp_grad_kernel<<<(kParams + 255) / 256, 256, 0, s>>>(gpart, kslices, grad);
+        e = cudaMemcpyAsync(grads_out, grad, sizeof(gm_mlp), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+      }
     } else {
       e = cudaMemcpy(net, d.p, sizeof(gm_mlp), cudaMemcpyDeviceToHost);
       net->steps = steps0 + total;
