@@ -11,6 +11,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <thread>
 #include <vector>
@@ -116,6 +117,11 @@ struct gm_ctx {
   gm::mlp::DevNet net;
   bool learned = false;
   int* mlp_err = nullptr;
+  int* mlp_err_host = nullptr;        // pinned: a call's copy of it
+  // gm_mlp_predict, gm_mlp_train: the caller's network on the device, kept
+  // between calls (0.8 MB), with the parameters it was last loaded from
+  gm::mlp::DevNet call_net;
+  std::unique_ptr<gm_mlp> call_params;
   // ragged batches: the layout of the last batch, its captured device work
   // and its resident-block limits per samples-per-lane class
   std::string batch_key;
@@ -162,6 +168,13 @@ gm_status ensure_buf(gm_ctx* ctx, const std::string& name, size_t bytes, void** 
   }
   *out = b.p;
   return GM_OK;
+}
+
+void drop_buf(gm_ctx* ctx, const std::string& name) {
+  auto it = ctx->bufs.find(name);
+  if (it == ctx->bufs.end()) return;
+  if (it->second.p) cudaFree(it->second.p);
+  ctx->bufs.erase(it);
 }
 
 // A host- or device-side argument staged onto the device.
@@ -342,6 +355,7 @@ gm_status gm_create(int device, size_t hbm_budget, gm_ctx** out) {
   if (cudaMalloc(&ctx->work2, sizeof(gm::WorkCounters)) != cudaSuccess) return GM_ERR_NOMEM;
   if (cudaMalloc(&ctx->mlp_err, sizeof(int) * 4) != cudaSuccess) return GM_ERR_NOMEM;
   cudaMemset(ctx->mlp_err, 0, sizeof(int) * 4);
+  if (cudaMallocHost(&ctx->mlp_err_host, sizeof(int)) != cudaSuccess) return GM_ERR_NOMEM;
   if (cudaStreamCreateWithFlags(&ctx->aux, cudaStreamNonBlocking) != cudaSuccess) return GM_ERR_CUDA;
   cudaEventCreateWithFlags(&ctx->evx0, cudaEventDisableTiming);
   cudaEventCreateWithFlags(&ctx->evx1, cudaEventDisableTiming);
@@ -367,7 +381,9 @@ gm_status gm_destroy(gm_ctx* ctx) {
   if (ctx->work) cudaFree(ctx->work);
   if (ctx->work2) cudaFree(ctx->work2);
   gm::mlp::devnet_destroy(&ctx->net);
+  gm::mlp::devnet_destroy(&ctx->call_net);
   if (ctx->mlp_err) cudaFree(ctx->mlp_err);
+  if (ctx->mlp_err_host) cudaFreeHost(ctx->mlp_err_host);
   if (ctx->batch_exec) cudaGraphExecDestroy(ctx->batch_exec);
   cudaEventDestroy(ctx->ev0);
   cudaEventDestroy(ctx->ev1);
@@ -409,6 +425,8 @@ gm_status gm_configure(gm_ctx* ctx, const gm_config* cfg) {
       return fail(ctx, GM_ERR_INVALID, "the network was made for another grid (its nl differs, or nl > 32)");
     if (cfg->lambda_per_pixel)
       return fail(ctx, GM_ERR_UNSUPPORTED, "the learned guess reads one grid, not per-pixel grids");
+    // freed first: that waits for inversions still reading the last network
+    gm::mlp::devnet_destroy(&ctx->net);
     cudaError_t e = gm::mlp::devnet_create(&ctx->net, net, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "learned initial guess upload");
@@ -537,6 +555,18 @@ static gm_status invert_chunks(gm_ctx* ctx, const gm::DevCfg& d, const gm::Inver
   if (e == cudaSuccess) e = cudaEventRecord(ctx->evx0, s);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->aux, ctx->evx0, 0);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "pipeline set-up");
+  auto copy_out = [&](int k) {
+    const int64_t a = cut(k), n = cut(k + 1) - a;
+    cudaError_t ce = cudaSuccess;
+    for (int o = 0; o < nouts && ce == cudaSuccess; ++o) {
+      const Arg& x = *outs[o];
+      if (!x.host || !x.dev) continue;
+      const size_t unit = x.bytes / (size_t)npix;
+      ce = cudaMemcpyAsync((char*)x.host + a * unit, (const char*)x.dev + a * unit, unit * n,
+                           cudaMemcpyDeviceToHost, (k & 1) ? ctx->aux : s);
+    }
+    return ce;
+  };
   cudaEventRecord(ctx->ev0, s);
   for (int k = 0; k < nch && e == cudaSuccess; ++k) {
     const int64_t a = cut(k), b = cut(k + 1), n = b - a;
@@ -571,14 +601,11 @@ static gm_status invert_chunks(gm_ctx* ctx, const gm::DevCfg& d, const gm::Inver
     ctx->stats.grid_blocks = (int)grid;
     ctx->stats.block_threads = geo.threads;
     ctx->stats.warps_per_block = geo.threads / 32;
-    for (int o = 0; o < nouts && e == cudaSuccess; ++o) {
-      const Arg& x = *outs[o];
-      if (!x.host || !x.dev) continue;
-      const size_t unit = x.bytes / (size_t)npix;
-      e = cudaMemcpyAsync((char*)x.host + a * unit, (const char*)x.dev + a * unit, unit * n,
-                          cudaMemcpyDeviceToHost, q);
-    }
+    // a chunk's outputs come back once the next chunk is on its way: a copy
+    // into pageable memory holds the host until the chunk is done
+    if (k > 0 && e == cudaSuccess) e = copy_out(k - 1);
   }
+  if (e == cudaSuccess) e = copy_out(nch - 1);
   if (e == cudaSuccess) e = cudaEventRecord(ctx->evx1, ctx->aux);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(s, ctx->evx1, 0);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "pipelined inversion");
@@ -1698,7 +1725,19 @@ static gm_status mlp_train_impl(gm_ctx* ctx, gm_mlp* net, const float* iquv, con
   ta.grads_only = grads_only;
   cudaMemsetAsync(ctx->mlp_err, 0, sizeof(int), s);
   const char* why = nullptr;
-  cudaError_t e = gm::mlp::train(net, ta, loss, grads, ctx->mlp_err, s, &why);
+  // one block of device memory for the call's buffers, kept while it is small
+  constexpr size_t kKeepBytes = (size_t)256 << 20;
+  const int64_t batch = grads_only ? n : (int64_t)o->batch;
+  void* ws = nullptr;
+  size_t need = 0;
+  if (batch > 0 && batch % gm::mlp::kTile == 0 && n >= batch && n <= (int64_t)1 << 31) {
+    need = gm::mlp::train_bytes(n, batch);
+    if ((st = ensure_buf(ctx, "mlp_ws", need, &ws)) != GM_OK) return st;
+  }
+  ctx->call_params.reset();
+  cudaError_t e =
+      gm::mlp::train(net, ta, ctx->call_net, ws, need, loss, grads, ctx->mlp_err, s, &why);
+  if (need > kKeepBytes) drop_buf(ctx, "mlp_ws");
   if (e == cudaErrorInvalidValue && why) return fail(ctx, GM_ERR_INVALID, why);
   if (e != cudaSuccess) return cuda_fail(ctx, e, why ? why : "training");
   return GM_OK;
@@ -1745,23 +1784,32 @@ gm_status gm_mlp_predict(gm_ctx* ctx, const gm_mlp* net, const float* iquv, int6
   if (reinterpret_cast<uintptr_t>(a_in.dev) & 15u)
     return fail(ctx, GM_ERR_INVALID, "device profiles must start on a 16-byte boundary");
   if ((st = stage_out(ctx, "pmodels", models, sizeof(double) * 11 * (size_t)n, &a_out)) != GM_OK) return st;
-  gm::mlp::DevNet d;
-  cudaError_t e = gm::mlp::devnet_create(&d, net, s);
+  // the network's device copy is loaded again only when its parameters differ
+  // from the last call's, compared value by value
+  cudaError_t e = cudaSuccess;
+  if (!ctx->call_params || std::memcmp(ctx->call_params.get(), net, sizeof(gm_mlp)) != 0) {
+    if (!ctx->call_params) ctx->call_params.reset(new (std::nothrow) gm_mlp);
+    if (ctx->call_params) std::memcpy(ctx->call_params.get(), net, sizeof(gm_mlp));
+    e = gm::mlp::devnet_create(&ctx->call_net, net, s);
+  }
   int fix[GM_NPAR];
   for (int i = 0; i < GM_NPAR; ++i) fix[i] = ctx->dev.fix[i];
   if (e == cudaSuccess) e = cudaMemsetAsync(ctx->mlp_err, 0, sizeof(int), s);
   if (e == cudaSuccess)
-    e = gm::mlp::predict(d, (const float*)a_in.dev, n, nl, ctx->cfg.init_model, fix, (double*)a_out.dev,
-                         ctx->mlp_err, s);
+    e = gm::mlp::predict(ctx->call_net, (const float*)a_in.dev, n, nl, ctx->cfg.init_model, fix,
+                         (double*)a_out.dev, ctx->mlp_err, s);
   if (e == cudaSuccess && (st = copy_back(ctx, a_out, s)) != GM_OK) {
-    gm::mlp::devnet_destroy(&d);
+    ctx->call_params.reset();
     return st;
   }
-  // the network's device copy is released with the call
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(ctx->mlp_err_host, ctx->mlp_err, sizeof(int), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  gm::mlp::devnet_destroy(&d);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "learned initial guess");
-  return learned_check(ctx);
+  if (e != cudaSuccess) {
+    ctx->call_params.reset();
+    return cuda_fail(ctx, e, "learned initial guess");
+  }
+  return *ctx->mlp_err_host ? learned_check(ctx) : GM_OK;
 }
 
 }  // extern "C"

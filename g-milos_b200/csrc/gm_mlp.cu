@@ -1389,21 +1389,53 @@ int sm_count() {
   return n > 0 ? n : 1;
 }
 
-// Device buffers of a training session, freed together.
-struct Buffers {
-  std::vector<void*> owned;
+// The buffers of a training call, carved from one block of device memory in
+// 256-byte steps; without memory it only adds up what they need.
+struct Carver {
+  char* base;
+  size_t used = 0;
   template <typename T>
-  cudaError_t get(T** p, size_t count) {
-    void* q = nullptr;
-    cudaError_t e = cudaMalloc(&q, sizeof(T) * count);
-    if (e == cudaSuccess) owned.push_back(q);
-    *p = static_cast<T*>(q);
-    return e;
-  }
-  ~Buffers() {
-    for (void* q : owned) cudaFree(q);
+  T* get(size_t count) {
+    T* p = base ? reinterpret_cast<T*>(base + used) : nullptr;
+    used += (sizeof(T) * count + 255) & ~(size_t)255;
+    return p;
   }
 };
+
+struct TrainBufs {
+  gm_mlp *grad, *m1, *m2;
+  uint16_t *x, *h1, *h2, *g1, *g2, *g3;
+  float *z, *y16, *loss, *gpart;
+  uint32_t* idx;
+  double2* part;
+  size_t bytes;
+};
+// one product block per SM; two (twice the slices) leave the products at
+// 13.5 us and make the optimiser sum twice as many partials, 8.7 us for 6.6
+int grad_slices(int64_t B, int sms) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(B / 64, sms / kWBlocks));
+}
+TrainBufs carve(void* base, int64_t n, int64_t B, int slices) {
+  Carver c{static_cast<char*>(base)};
+  TrainBufs b{};
+  b.grad = c.get<gm_mlp>(1);
+  b.m1 = c.get<gm_mlp>(1);
+  b.m2 = c.get<gm_mlp>(1);
+  b.x = c.get<uint16_t>((size_t)B * kIn);
+  b.h1 = c.get<uint16_t>((size_t)B * kHid);
+  b.h2 = c.get<uint16_t>((size_t)B * kHid);
+  b.g1 = c.get<uint16_t>((size_t)B * kHid);
+  b.g2 = c.get<uint16_t>((size_t)B * kHid);
+  b.g3 = c.get<uint16_t>((size_t)B * kG);
+  b.z = c.get<float>((size_t)B * kHid);
+  b.y16 = c.get<float>((size_t)n * 16);
+  b.idx = c.get<uint32_t>((size_t)n);
+  b.loss = c.get<float>(1);
+  b.part = c.get<double2>((size_t)kMomBlocks * kMom);
+  b.gpart = c.get<float>((size_t)slices * kPartStride);
+  b.bytes = c.used;
+  return b;
+}
 
 }  // namespace
 
@@ -1425,25 +1457,36 @@ void init_net(gm_mlp* net, int nl, uint64_t seed) {
   fill(&net->w3[0][0], kOut, kHid, kHid, 0.1f);   // outputs start near the mean
 }
 
-cudaError_t devnet_create(DevNet* d, const gm_mlp* host, cudaStream_t s) {
-  devnet_destroy(d);
-  cudaError_t e = cudaMalloc(&d->p, sizeof(gm_mlp));
-  if (e == cudaSuccess) e = cudaMalloc(&d->pack, sizeof(uint16_t) * kPackElems);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d->pack, 0, sizeof(uint16_t) * kPackElems, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d->p, host, sizeof(gm_mlp), cudaMemcpyHostToDevice, s);
+cudaError_t devnet_load(DevNet* d, const gm_mlp* host, cudaStream_t s) {
+  cudaError_t e = cudaMemcpyAsync(d->p, host, sizeof(gm_mlp), cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return e;
   mlp_pack_kernel<<<256, 256, 0, s>>>(d->p, d->pack);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  NetMaps nm;
-  if (!net_maps(d->pack, &nm)) return cudaErrorInvalidValue;
-  d->mw1 = nm.m[kMapW1];
-  d->mw2 = nm.m[kMapW2];
-  d->mw3 = nm.m[kMapW3];
-  d->mw2t = nm.m[kMapW2t];
-  d->mw3t = nm.m[kMapW3t];
   d->nl = host->nl;
-  return cudaSuccess;
+  return cudaGetLastError();
+}
+
+cudaError_t devnet_create(DevNet* d, const gm_mlp* host, cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
+  if (!d->p) {
+    DevNet n;
+    e = cudaMalloc(&n.p, sizeof(gm_mlp));
+    if (e == cudaSuccess) e = cudaMalloc(&n.pack, sizeof(uint16_t) * kPackElems);
+    // the copies' padding stays zero
+    if (e == cudaSuccess) e = cudaMemsetAsync(n.pack, 0, sizeof(uint16_t) * kPackElems, s);
+    NetMaps nm;
+    if (e == cudaSuccess && !net_maps(n.pack, &nm)) e = cudaErrorInvalidValue;
+    if (e != cudaSuccess) {
+      devnet_destroy(&n);
+      return e;
+    }
+    n.mw1 = nm.m[kMapW1];
+    n.mw2 = nm.m[kMapW2];
+    n.mw3 = nm.m[kMapW3];
+    n.mw2t = nm.m[kMapW2t];
+    n.mw3t = nm.m[kMapW3t];
+    *d = n;
+  }
+  return devnet_load(d, host, s);
 }
 
 void devnet_destroy(DevNet* d) {
@@ -1484,8 +1527,12 @@ cudaError_t predict(const DevNet& d, const float* iquv, int64_t n, int nl, const
   return cudaGetLastError();
 }
 
-cudaError_t train(gm_mlp* net, const TrainArgs& a, float* loss_out, gm_mlp* grads_out, int* err, cudaStream_t s,
-                  const char** why) {
+size_t train_bytes(int64_t n, int64_t batch) {
+  return carve(nullptr, n, batch, grad_slices(batch, sm_count())).bytes;
+}
+
+cudaError_t train(gm_mlp* net, const TrainArgs& a, DevNet& d, void* ws, size_t ws_bytes, float* loss_out,
+                  gm_mlp* grads_out, int* err, cudaStream_t s, const char** why) {
   auto fail = [&](const char* w, cudaError_t e) {
     if (why) *why = w;
     return e;
@@ -1498,36 +1545,19 @@ cudaError_t train(gm_mlp* net, const TrainArgs& a, float* loss_out, gm_mlp* grad
   if (!err) return fail("no error word", cudaErrorInvalidValue);
   if (reinterpret_cast<uintptr_t>(a.iquv) & 15u)
     return fail("the profiles must start on a 16-byte boundary", cudaErrorInvalidValue);
-  Buffers buf;
-  DevNet d;
-  cudaError_t e = devnet_create(&d, net, s);
-  if (e != cudaSuccess) {
-    devnet_destroy(&d);
-    return fail("network upload", e);
-  }
-  gm_mlp *grad = nullptr, *m1 = nullptr, *m2 = nullptr;
-  uint16_t *x = nullptr, *h1 = nullptr, *h2 = nullptr, *g1 = nullptr, *g2 = nullptr, *g3 = nullptr;
-  float *z = nullptr, *y16 = nullptr, *loss = nullptr, *gpart = nullptr;
-  uint32_t* idx = nullptr;
-  double2* part = nullptr;
   const int64_t n = a.n;
   const int sms = sm_count();
   const int64_t tiles = B / kTile;
   const int tgrid = (int)std::min<int64_t>(tiles, sms);
-  // one product block per SM; two (twice the slices) leave the products at
-  // 13.5 us and make the optimiser sum twice as many partials, 8.7 us for 6.6
-  const int kslices = (int)std::max<int64_t>(1, std::min<int64_t>(B / 64, sms / kWBlocks));
-  if ((e = buf.get(&grad, 1)) != cudaSuccess || (e = buf.get(&m1, 1)) != cudaSuccess ||
-      (e = buf.get(&m2, 1)) != cudaSuccess || (e = buf.get(&x, (size_t)B * kIn)) != cudaSuccess ||
-      (e = buf.get(&h1, (size_t)B * kHid)) != cudaSuccess || (e = buf.get(&h2, (size_t)B * kHid)) != cudaSuccess ||
-      (e = buf.get(&g1, (size_t)B * kHid)) != cudaSuccess || (e = buf.get(&g2, (size_t)B * kHid)) != cudaSuccess ||
-      (e = buf.get(&g3, (size_t)B * kG)) != cudaSuccess || (e = buf.get(&z, (size_t)B * kHid)) != cudaSuccess ||
-      (e = buf.get(&y16, (size_t)n * 16)) != cudaSuccess || (e = buf.get(&idx, (size_t)n)) != cudaSuccess ||
-      (e = buf.get(&loss, 1)) != cudaSuccess || (e = buf.get(&part, (size_t)kMomBlocks * kMom)) != cudaSuccess ||
-      (e = buf.get(&gpart, (size_t)kslices * kPartStride)) != cudaSuccess) {
-    devnet_destroy(&d);
-    return fail("device allocation", e);
-  }
+  const int kslices = grad_slices(B, sms);
+  const TrainBufs buf = carve(ws, n, B, kslices);
+  if (!ws || ws_bytes < buf.bytes) return fail("no workspace", cudaErrorInvalidValue);
+  gm_mlp *grad = buf.grad, *m1 = buf.m1, *m2 = buf.m2;
+  uint16_t *x = buf.x, *h1 = buf.h1, *h2 = buf.h2, *g1 = buf.g1, *g2 = buf.g2, *g3 = buf.g3;
+  float *z = buf.z, *y16 = buf.y16, *loss = buf.loss, *gpart = buf.gpart;
+  uint32_t* idx = buf.idx;
+  cudaError_t e = devnet_create(&d, net, s);
+  if (e != cudaSuccess) return fail("network upload", e);
   cudaMemsetAsync(grad, 0, sizeof(gm_mlp), s);
   cudaMemsetAsync(m1, 0, sizeof(gm_mlp), s);
   cudaMemsetAsync(m2, 0, sizeof(gm_mlp), s);
@@ -1540,23 +1570,17 @@ cudaError_t train(gm_mlp* net, const TrainArgs& a, float* loss_out, gm_mlp* grad
               make_map(&wm.a[0], g1, kHid, B, 64) && make_map(&wm.b[0], x, kIn, B, 64) &&
               make_map(&wm.a[1], g2, kHid, B, 64) && make_map(&wm.b[1], h1, kHid, B, 64) &&
               make_map(&wm.a[2], h2, kHid, B, 64) && make_map(&wm.b[2], g3, kG, B, 64);
-  if (!maps) {
-    devnet_destroy(&d);
-    return fail("tensor-map encoding", cudaErrorInvalidValue);
-  }
+  if (!maps) return fail("tensor-map encoding", cudaErrorInvalidValue);
   if (net->steps == 0 && !a.grads_only) {
     const int64_t m = std::min<int64_t>(n, 65536);
-    mlp_moments_kernel<<<kMomBlocks, kMomThreads, 0, s>>>(a.iquv, a.truth, m, a.nl, part);
-    mlp_standardise_kernel<<<1, kMom, 0, s>>>(part, kMomBlocks, m, a.nl, d.p);
+    mlp_moments_kernel<<<kMomBlocks, kMomThreads, 0, s>>>(a.iquv, a.truth, m, a.nl, buf.part);
+    mlp_standardise_kernel<<<1, kMom, 0, s>>>(buf.part, kMomBlocks, m, a.nl, d.p);
   }
   mlp_targets_kernel<<<1024, 256, 0, s>>>(a.truth, n, d.p, y16);
   e = cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(mlp_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgradSmem);
-  if (e != cudaSuccess) {
-    devnet_destroy(&d);
-    return fail("kernel attributes", e);
-  }
+  if (e != cudaSuccess) return fail("kernel attributes", e);
   const int epochs = a.grads_only ? 1 : std::max(1, a.epochs);
   const int64_t steps_per_epoch = n / B;
   const int64_t total = steps_per_epoch * epochs;
@@ -1625,7 +1649,6 @@ cudaError_t train(gm_mlp* net, const TrainArgs& a, float* loss_out, gm_mlp* grad
       net->steps = steps0 + total;
     }
   }
-  devnet_destroy(&d);
   return e == cudaSuccess ? e : fail(code ? "a training kernel gave up waiting" : "training", e);
 }
 

@@ -37,8 +37,8 @@ constexpr size_t kW2tb = kW3b + (size_t)kOut16 * kHid;      // [256][256] transp
 constexpr size_t kW3tb = kW2tb + (size_t)kHid * kHid;       // [256][64]  transposed w3 (cols >= 9 zero)
 constexpr size_t kPackElems = kW3tb + (size_t)kHid * kG;
 
-// Set up / release a device network from host parameters (copy, BF16 pack,
-// descriptors); stream-ordered.
+// Load host parameters into a device network (copy, BF16 pack), allocating it
+// and its descriptors the first time; release it.  Stream-ordered.
 cudaError_t devnet_create(DevNet* d, const gm_mlp* host, cudaStream_t s);
 void devnet_destroy(DevNet* d);
 
@@ -63,8 +63,11 @@ struct TrainArgs {
   uint64_t seed;
   bool grads_only;
 };
-cudaError_t train(gm_mlp* net, const TrainArgs& a, float* loss, gm_mlp* grads, int* err, cudaStream_t s,
-                  const char** why);
+// d: a device network the call may overwrite (allocated as needed); ws: at
+// least train_bytes(n, batch) bytes of device memory.
+size_t train_bytes(int64_t n, int64_t batch);
+cudaError_t train(gm_mlp* net, const TrainArgs& a, DevNet& d, void* ws, size_t ws_bytes, float* loss, gm_mlp* grads,
+                  int* err, cudaStream_t s, const char** why);
 
 // A fresh network (host only).
 void init_net(gm_mlp* net, int nl, uint64_t seed);
