@@ -179,6 +179,18 @@ struct Jacobi11 {
   double V[S11 ? 2 : 1][S11 ? 144 : 1];
 };
 
+// circ_rows convolves circ_batch rows at a time, each on circ_lanes lanes with
+// kCircOut neighbouring outputs a lane; an odd number of outputs keeps the
+// samples that a row's lanes read at once in distinct banks.
+constexpr int kCircOut = 5;
+template <int LPL>
+__host__ __device__ constexpr int circ_batch() { return 4 / LPL; }
+template <int LPL>
+__host__ __device__ constexpr int circ_lanes() { return (32 * LPL + kCircOut - 1) / kCircOut; }
+template <int LPL>
+__host__ __device__ constexpr int circ_pitch() { return 64 * LPL + kCircOut; }   // two copies and 4 samples more
+static_assert(circ_lanes<1>() * circ_batch<1>() <= 32 && circ_lanes<2>() * circ_batch<2>() <= 32, "one warp");
+
 // Warp-private shared memory: the half-warp solve's space, then the models and
 // what a synthesis touches, then the staged rows.  The wave kernels back only
 // a part of it (a warp's stride in their shared memory): a trial the rows' first
@@ -199,8 +211,10 @@ struct WarpSmem {
   alignas(16) double m[11];   // current (last accepted) model: the reference's initModel
   double t[11];          // trial model, persistent like the reference's `model`
   float ic[NR];          // continuum about which each staged I row is reflected
-  double gk[Variant<V>::MAC ? kMaxNl : 1];   // macroturbulence kernel (PSF folded in)
-  double gd[Variant<V>::MAC ? kMaxNl : 1];   // its derivative with respect to v_mac
+  double gk[Variant<V>::MAC ? 64 * LPL : 1];   // macroturbulence kernel (PSF folded in)
+  double gd[Variant<V>::MAC ? 64 * LPL : 1];   // its derivative with respect to v_mac
+  // rows on their way through a circular convolution, in double
+  double xd[Variant<V>::MAC ? circ_batch<LPL>() * circ_pitch<LPL>() : 1];
   double dd[S11 ? 12 : 1];                   // FP64 step of the 11-term solve
   double b11[S11 ? 12 : 1], z11[S11 ? 12 : 1];
   double c11[S11 ? 6 : 1], s11[S11 ? 6 : 1]; // the step's rotations
@@ -338,14 +352,30 @@ __device__ __forceinline__ void psf_rows(WarpSmem<LPL, V>& sm, const DevCfg& c, 
 // derivative with respect to v_mac, g / v_mac * (x^2 - 1) (me_der.cu:122-129),
 // in sm.gd.  With a PSF both are then correlated with it in double, zero
 // padded about nl/2 (direct_convolution_double, convolution.cu:120-151;
-// mil_sinrf.cu:105-107, me_der.cu:131-136).  lamp: the pixel's own
-// wavelengths, or null for the configured grid.
+// mil_sinrf.cu:105-107, me_der.cu:131-136), its taps read from the block's
+// copy.  Out of line, as circ_rows: the synthesis and the response functions
+// share one copy of the code.
+// The wavelength offsets of this lane's samples from sample nl/2.
+template <int LPL>
+struct MacOffsets {
+  double x[LPL];
+};
+template <int LPL>
+__device__ __forceinline__ MacOffsets<LPL> mac_offsets(const DevCfg& c, const double* lamp, int lane) {
+  MacOffsets<LPL> o;
+  const double lc = lamp ? lamp[c.nl >> 1] : c.lam[c.nl >> 1];
+#pragma unroll
+  for (int k = 0; k < LPL; ++k) {
+    const int l = lane + 32 * k;
+    o.x[k] = l < c.nl ? (lamp ? lamp[l] : c.lam[l]) - lc : 0.0;
+  }
+  return o;
+}
 template <int LPL, int V>
-__device__ __forceinline__ void mac_kernels(const DevCfg& c, WarpSmem<LPL, V>& sm, double mac,
-                                            int lane, bool deriv, const double* lamp) {
-  const int nl = c.nl, half = nl >> 1;
-  const double ild = (c.lambda0 * mac) / kVlight;
-  const double lc = lamp ? lamp[half] : c.lam[half];
+__device__ __noinline__ void mac_kernels(WarpSmem<LPL, V>& sm, int nl, bool use_psf, MacOffsets<LPL> off,
+                                         double lambda0, double mac, int lane, bool deriv) {
+  const int half = nl >> 1;
+  const double ild = (lambda0 * mac) / kVlight;
   double g[LPL], x2[LPL], part = 0.0;
 #pragma unroll
   for (int k = 0; k < LPL; ++k) {
@@ -353,7 +383,7 @@ __device__ __forceinline__ void mac_kernels(const DevCfg& c, WarpSmem<LPL, V>& s
     g[k] = 0.0;
     x2[k] = 0.0;
     if (l < nl) {
-      const double x = ((lamp ? lamp[l] : c.lam[l]) - lc) / ild;
+      const double x = off.x[k] / ild;
       const double term = (x * x) / 2;
       g[k] = term < 1e30 ? exp(-term) : 0.0;
       x2[k] = x * x;
@@ -361,40 +391,51 @@ __device__ __forceinline__ void mac_kernels(const DevCfg& c, WarpSmem<LPL, V>& s
     }
   }
   const double sum = warp_sum_d(part);
+  double gn[LPL], gp[LPL];
 #pragma unroll
   for (int k = 0; k < LPL; ++k) {
-    const int l = lane + 32 * k;
-    if (l < nl) {
-      const double gn = g[k] / sum;
-      sm.gk[l] = gn;
-      if (deriv) sm.gd[l] = gn / mac * (x2[k] - 1.0);
-    }
+    gn[k] = g[k] / sum;
+    gp[k] = deriv ? gn[k] / mac * (x2[k] - 1.0) : 0.0;
   }
-  __syncwarp();
-  if (!c.use_psf) return;
-  double og[LPL], od[LPL];
+  if (use_psf) {
+    // the kernels at [half, half + nl) of 2 nl zeros: the sums need no bounds
 #pragma unroll
-  for (int k = 0; k < LPL; ++k) {
-    const int l = lane + 32 * k;
-    double a = 0.0, b = 0.0;
-    if (l < nl) {
-      for (int j = 0; j < nl; ++j) {
-        const int idx = l + j - half;
-        if (idx < 0 || idx >= nl) continue;
-        a += c.psfd[j] * sm.gk[idx];
-        if (deriv) b += c.psfd[j] * sm.gd[idx];
+    for (int k = 0; k < 2 * LPL; ++k) {
+      sm.gk[lane + 32 * k] = 0.0;
+      if (deriv) sm.gd[lane + 32 * k] = 0.0;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < LPL; ++k) {
+      const int l = lane + 32 * k;
+      if (l < nl) {
+        sm.gk[half + l] = gn[k];
+        if (deriv) sm.gd[half + l] = gp[k];
+      }
+      gn[k] = 0.0;
+      gp[k] = 0.0;
+    }
+    __syncwarp();
+#pragma unroll 2
+    for (int j = 0; j < nl; ++j) {
+      const double h = block_taps()[tap_off<LPL>() + j];
+#pragma unroll
+      for (int k = 0; k < LPL; ++k) {
+        const int l = lane + 32 * k;
+        if (l < nl) {
+          gn[k] += h * sm.gk[l + j];
+          if (deriv) gp[k] += h * sm.gd[l + j];
+        }
       }
     }
-    og[k] = a;
-    od[k] = b;
+    __syncwarp();
   }
-  __syncwarp();
 #pragma unroll
   for (int k = 0; k < LPL; ++k) {
     const int l = lane + 32 * k;
     if (l < nl) {
-      sm.gk[l] = og[k];
-      if (deriv) sm.gd[l] = od[k];
+      sm.gk[l] = gn[k];
+      if (deriv) sm.gd[l] = gp[k];
     }
   }
   __syncwarp();
@@ -405,37 +446,80 @@ __device__ __forceinline__ void mac_kernels(const DevCfg& c, WarpSmem<LPL, V>& s
 // rotated so that sample nl/2 is the zero lag (convCircular,
 // convolution.cu:251-279): output m takes the circular sum at index
 // (m + nl/2) mod nl.  The caller syncs the warp after staging.
+//
+// The rows are converted to double once and laid out twice over, so that no
+// index wraps.  A lane forms five neighbouring outputs of one row: every tap
+// takes one new sample for five products, in a window that moves through
+// registers (a sample loaded for each product left the shared-memory port the
+// bound, 270 cycles for four rows where this takes 90), and each output is its
+// own chain in the order of j.  Out of line: the synthesis and the response
+// functions share the code, the kernels that reach it being bound by
+// instruction fetch.
 template <int LPL, int V>
-__device__ __forceinline__ void circ_rows(WarpSmem<LPL, V>& sm, const DevCfg& c, uint64_t mask,
-                                          const double* h, int lane) {
-  const int nl = c.nl, half = nl >> 1;
+__device__ __noinline__ void circ_rows(WarpSmem<LPL, V>& sm, int nl, uint64_t mask, const double* h, int lane) {
+  constexpr int N = circ_batch<LPL>(), L = circ_lanes<LPL>(), T = kCircOut, PITCH = circ_pitch<LPL>();
+  const int half = nl >> 1;
+  const int q = lane / L, m0 = T * (lane - q * L);
+  // sample (m + half - j) mod nl of output m = m0 + c at xs[c - j]; the last
+  // tap's xs[-j - 1], not used, is still inside the row
+  const double* xs = sm.xd + q * PITCH + (m0 + half >= nl ? m0 + half : m0 + half + nl);
+#pragma unroll 1
   while (mask) {
-    const int r = __ffsll((long long)mask) - 1;
-    mask &= mask - 1;
-    const float* x = sm.rows[r];
-    float out[LPL];
+    int mine = -1;
 #pragma unroll
-    for (int k = 0; k < LPL; ++k) {
-      const int mo = lane + 32 * k;
-      double a = 0.0;
-      if (mo < nl) {
-        int idx = mo + half;
-        if (idx >= nl) idx -= nl;
-        for (int j = 0; j < nl; ++j) {
-          a += h[j] * (double)x[idx];
-          idx = (idx == 0) ? nl - 1 : idx - 1;
+    for (int p = 0; p < N; ++p) {
+      if (mask) {
+        const int r = __ffsll((long long)mask) - 1;
+        mask &= mask - 1;
+        if (p == q) mine = r;
+#pragma unroll
+        for (int k = 0; k < LPL; ++k) {
+          const int l = lane + 32 * k;
+          if (l < nl) {
+            const double x = (double)sm.rows[r][l];
+            double* d = sm.xd + p * PITCH + l;
+            d[0] = x;
+            d[nl] = x;
+            if (l < T - 1) d[2 * nl] = x;
+          }
         }
       }
-      out[k] = (float)a;
     }
     __syncwarp();
+    if (mine >= 0 && m0 < nl) {
+      double a[T], x[T];
 #pragma unroll
-    for (int k = 0; k < LPL; ++k) {
-      const int mo = lane + 32 * k;
-      if (mo < nl) sm.rows[r][mo] = out[k];
+      for (int c = 0; c < T; ++c) {
+        a[c] = 0.0;
+        x[c] = xs[c];
+      }
+      // the window's samples xs[c - j - u] in x[(c + T - u) % T]
+      int j = 0;
+#pragma unroll 1
+      for (; j + T <= nl; j += T) {
+#pragma unroll
+        for (int u = 0; u < T; ++u) {
+          const double hj = h[j + u];
+#pragma unroll
+          for (int c = 0; c < T; ++c) a[c] += hj * x[(c + T - u) % T];
+          x[T - 1 - u] = xs[-j - u - 1];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < T - 1; ++u) {
+        if (j + u < nl) {
+          const double hj = h[j + u];
+#pragma unroll
+          for (int c = 0; c < T; ++c) a[c] += hj * x[(c + T - u) % T];
+          x[T - 1 - u] = xs[-j - u - 1];
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < T; ++c)
+        if (m0 + c < nl) sm.rows[mine][m0 + c] = (float)a[c];
     }
+    __syncwarp();
   }
-  __syncwarp();
 }
 
 // --------------------------------------------------------------- synthesis
@@ -542,7 +626,7 @@ __device__ __forceinline__ void synth_lane(const DevCfg& c, const double* m, con
   if (mac_on) {
     // macroturbulence with the PSF folded into its kernel; the PSF is not
     // applied again (mil_sinrf.cu:101-130)
-    mac_kernels<LPL, V>(c, sm, m[MAC], lane, false, lamp);
+    mac_kernels<LPL, V>(sm, c.nl, c.use_psf != 0, mac_offsets<LPL>(c, lamp, lane), c.lambda0, m[MAC], lane, false);
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
       float row[LPL];
@@ -551,7 +635,7 @@ __device__ __forceinline__ void synth_lane(const DevCfg& c, const double* m, con
       put_row<LPL, V>(sm, s, row, c.nl, lane, false);
     }
     __syncwarp();
-    circ_rows<LPL, V>(sm, c, 0xfull, sm.gk, lane);
+    circ_rows<LPL, V>(sm, c.nl, 0xfull, sm.gk, lane);
 #pragma unroll
     for (int k = 0; k < LPL; ++k)
 #pragma unroll
@@ -766,7 +850,7 @@ __device__ __forceinline__ void rf_rows(const DevCfg& c, const double* m, const 
       // macroturbulence (me_der.cu:117-156): the v_mac RF is the profile
       // before convolution through the kernel's derivative; every other
       // staged RF goes through the kernel (PSF folded into both)
-      mac_kernels<LPL, V>(c, sm, m[MAC], lane, true, lamp);
+      mac_kernels<LPL, V>(sm, nl, c.use_psf != 0, mac_offsets<LPL>(c, lamp, lane), c.lambda0, m[MAC], lane, true);
 #pragma unroll
       for (int s = 0; s < 4; ++s) {
         float row[LPL];
@@ -775,8 +859,8 @@ __device__ __forceinline__ void rf_rows(const DevCfg& c, const double* m, const 
         put_row<LPL, V>(sm, mac_row(s), row, nl, lane, false);
       }
       __syncwarp();
-      circ_rows<LPL, V>(sm, c, 0xfull << kRows, sm.gd, lane);
-      circ_rows<LPL, V>(sm, c, (uint64_t)mask, sm.gk, lane);
+      circ_rows<LPL, V>(sm, nl, 0xfull << kRows, sm.gd, lane);
+      circ_rows<LPL, V>(sm, nl, (uint64_t)mask, sm.gk, lane);
     }
   } else if (c.use_psf) {
     // reflect the I rows about max(first, last) (me_der.cu:167-176)
@@ -1229,6 +1313,15 @@ __host__ __device__ constexpr SolvePlans solve_plans() {
 }
 static __device__ const SolvePlans g_solve_plans[2] = {solve_plans<1>(), solve_plans<2>()};
 
+// The rotations' products and multiply-adds are written out, so that every
+// form of the solve rounds alike: the first product fused, the second rounded.
+__device__ __forceinline__ float mul_sub(float a, float b, float c, float d) {   // a b - c d
+  return __fmaf_rn(a, b, -__fmul_rn(c, d));
+}
+__device__ __forceinline__ float mul_add(float a, float b, float c, float d) {   // a b + c d
+  return __fmaf_rn(a, b, __fmul_rn(c, d));
+}
+
 // Solves for damping 1 + flambda into sm.vec[0][0] and, with two solves per
 // call, for 1 + flambda2 into sm.vec[1][0].  `accurate` (the numerics mode)
 // is a template parameter and the solve an out-of-line function: a runtime
@@ -1239,22 +1332,12 @@ template <int LPL, int V, bool accurate>
 __device__ __noinline__ void solve10(WarpSmem<LPL, V>& sm, const SolvePlan& pl, float flambda,
                                         float flambda2, int lane) {
   constexpr int NS = Variant<V>::SOLVES, G = 32 / NS;
-  // The plan's indices (all below 256) packed one byte each into three
-  // registers: read through the reference, every store to the shared-memory
-  // blocks might alias the plan and each step would reload it from local
-  // memory, and unpacked the eleven values spill (+3.6 % pixels/s packed).
-  const unsigned w0 = (unsigned)pl.src | (unsigned)pl.d00 << 8 | (unsigned)pl.d01 << 16 | (unsigned)pl.d10 << 24;
-  const unsigned w1 = (unsigned)pl.d11 | (unsigned)pl.vin << 8 | (unsigned)pl.vout0 << 16 | (unsigned)pl.vout1 << 24;
-  const unsigned w2 = (unsigned)pl.p | (unsigned)(pl.base + pl.p) << 8 | (unsigned)(pl.base + pl.q) << 16 |
-                     (unsigned)pl.wdiag << 24;
   const unsigned initpack = pl.initpack;
-  auto at = [](unsigned w, int i) { return (int)((w >> (8 * i)) & 0xffu); };
   const int h = NS == 2 ? lane >> 4 : 0;
   const int g = lane & (G - 1);
   // damped matrix (diagonal x (1 + lambda), milosUtils.cu:648-652)
   const double damp = 1.0 + (double)(h ? flambda2 : flambda);
   float* A = &sm.A[h * kSolveH];
-  float* B = A + kSolveB;
 #pragma unroll
   for (int e = 0; e < 2 * NS; ++e) {
     const unsigned b = (initpack >> (8 * e)) & 0xffu;
@@ -1264,60 +1347,75 @@ __device__ __noinline__ void solve10(WarpSmem<LPL, V>& sm, const SolvePlan& pl, 
     }
   }
   float* va = &sm.vec[h][0][0];
-  float* vb = &sm.vec[h][1][0];
   if (g < 10) va[g] = sm.beta[g];
   __syncwarp();
 
   const float quarter = (float)(kPi / 4);
   const float qclamp = __fdividef((float)kPi, 4.f);
   const bool diag = g < 5, active = g < 15;
+  // this lane's places, taken out of the plan once; the two buffers are a
+  // constant apart, so a step's addresses need no arithmetic when the steps run
+  // in pairs, one in each direction
+  const float* src = A + pl.src;
+  float *const d00 = A + pl.d00, *const d01 = A + pl.d01, *const d10 = A + pl.d10, *const d11 = A + pl.d11;
+  const float* vsrc = va + pl.vin;
+  float *const v0 = va + pl.vout0, *const v1 = va + pl.vout1;
+  const int pr = pl.base + pl.p, pq = pl.base + pl.q;
+  float* rc = &sm.cs[h][0][diag ? g : 0];
+  float* rs = &sm.sn[h][0][diag ? g : 0];
 #pragma unroll 1
-  for (int step = 0; step < 18; ++step) {
-    const float4 blk = *reinterpret_cast<const float4*>(A + at(w0, 0));
-    const float m00 = blk.x, m01 = blk.y, m11 = blk.w;
-    const float m10 = diag ? m01 : blk.z;
-    const float b0 = va[at(w1, 1)], b1 = va[at(w1, 1) + 1];
-    float th;
-    if (m00 == m11) {
-      th = quarter;
-    } else {
-      const float arc = accurate ? (2.f * m01) / (m11 - m00) : __fdividef(2.f * m01, m11 - m00);
-      th = accurate ? atanf(arc) / 2.f : __fdividef(atanf(arc), 2.f);
-      th = fminf(fmaxf(th, -qclamp), qclamp);
+  for (int step = 0; step < 18; step += 2) {
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      // from the first buffers to the second, then back
+      constexpr int VB = 12;
+      const int ra = half ? kSolveB : 0, wa = half ? 0 : kSolveB, rv = half ? VB : 0, wv = half ? 0 : VB;
+      const float4 blk = *reinterpret_cast<const float4*>(src + ra);
+      const float m00 = blk.x, m01 = blk.y, m11 = blk.w;
+      const float m10 = diag ? m01 : blk.z;
+      const float b0 = vsrc[rv], b1 = vsrc[rv + 1];
+      float th;
+      if (m00 == m11) {
+        th = quarter;
+      } else {
+        const float arc = accurate ? (2.f * m01) / (m11 - m00) : __fdividef(2.f * m01, m11 - m00);
+        th = accurate ? atanf(arc) / 2.f : __fdividef(atanf(arc), 2.f);
+        th = fminf(fmaxf(th, -qclamp), qclamp);
+      }
+      float sn, cs;
+      sincos_mode(th, &sn, &cs, accurate);
+      if (diag) {
+        rc[0] = cs;
+        rs[0] = sn;
+      }
+      rc += 5;
+      rs += 5;
+      const float cr = __shfl_sync(kFull, cs, pr), sr = __shfl_sync(kFull, sn, pr);
+      const float cc = __shfl_sync(kFull, cs, pq), sc = __shfl_sync(kFull, sn, pq);
+      const float t0 = mul_sub(m00, cr, m10, sr), t1 = mul_add(m10, cr, m00, sr);
+      const float u0 = mul_sub(m01, cr, m11, sr), u1 = mul_add(m11, cr, m01, sr);
+      const float n00 = mul_sub(t0, cc, u0, sc), n11 = mul_add(t1, sc, u1, cc);
+      const float n01 = diag ? 0.f : mul_add(t0, sc, u0, cc);
+      const float n10 = mul_sub(t1, cc, u1, sc);
+      if (active) {
+        d00[wa] = n00;
+        d01[wa] = n01;
+        if (!diag) d10[wa] = n10;   // a diagonal block's two off-diagonal entries are one
+        d11[wa] = n11;
+      }
+      if (diag) {
+        v0[wv] = mul_sub(cs, b0, sn, b1);
+        v1[wv] = mul_add(sn, b0, cs, b1);
+      }
+      __syncwarp();
     }
-    float sn, cs;
-    sincos_mode(th, &sn, &cs, accurate);
-    if (diag) {
-      sm.cs[h][step][g] = cs;
-      sm.sn[h][step][g] = sn;
-    }
-    const float cr = __shfl_sync(kFull, cs, at(w2, 1)), sr = __shfl_sync(kFull, sn, at(w2, 1));
-    const float cc = __shfl_sync(kFull, cs, at(w2, 2)), sc = __shfl_sync(kFull, sn, at(w2, 2));
-    const float t0 = m00 * cr - m10 * sr, t1 = m00 * sr + m10 * cr;
-    const float u0 = m01 * cr - m11 * sr, u1 = m01 * sr + m11 * cr;
-    const float n00 = t0 * cc - u0 * sc, n11 = t1 * sc + u1 * cc;
-    const float n01 = diag ? 0.f : t0 * sc + u0 * cc;
-    const float n10 = diag ? 0.f : t1 * cc - u1 * sc;
-    if (active) {
-      B[at(w0, 1)] = n00;
-      B[at(w0, 2)] = n01;
-      if (!diag) B[at(w0, 3)] = n10;   // a diagonal block's two off-diagonal entries are one
-      B[at(w1, 0)] = n11;
-    }
-    if (diag) {
-      vb[at(w1, 2)] = cs * b0 - sn * b1;
-      vb[at(w1, 3)] = sn * b0 + cs * b1;
-    }
-    __syncwarp();
-    float* tA = A; A = B; B = tA;
-    float* tv = va; va = vb; vb = tv;
   }
   // 18 steps: the final matrix and vector are back in the first buffers, in
   // the original index order.  z = (V^T beta) / w with the |w| <= 1e-12 cut,
   // component g in group lane g's register.
   float y = 0.f;
   if (g < 10) {
-    const float w = A[at(w2, 3)];
+    const float w = A[pl.wdiag];
     const float inv = ((double)fabsf(w) > 1e-12) ? (1.f / w) : 0.f;
     y = va[g] * inv;
   }
@@ -1335,7 +1433,7 @@ __device__ __noinline__ void solve10(WarpSmem<LPL, V>& sm, const SolvePlan& pl, 
   for (int step = 17; step >= 0; --step) {
     const float y0 = __shfl_sync(kFull, y, y0_lane), y1 = __shfl_sync(kFull, y, y1_lane);
     const float cs = sm.cs[h][step][k], sn = sm.sn[h][step][k];
-    y = second ? -sn * y0 + cs * y1 : cs * y0 + sn * y1;
+    y = second ? mul_sub(cs, y1, sn, y0) : mul_add(cs, y0, sn, y1);
   }
   if (g < 10) sm.vec[h][0][g] = y;
   __syncwarp();
@@ -1343,18 +1441,10 @@ __device__ __noinline__ void solve10(WarpSmem<LPL, V>& sm, const SolvePlan& pl, 
 
 // --------------------------------------------------------------- 10x10 solve, one thread each
 // solve10's arithmetic with a whole system in one thread's registers: the
-// same 18 steps on the same 2x2 blocks in the same order, every product and
-// multiply-add written out as solve10's expressions compile (which product
-// of a pair is fused and which is rounded first), so a step's result is that
-// of solve10 bit for bit.  What it saves is lanes: solve10's half-warp forms each angle
+// same 18 steps on the same 2x2 blocks in the same order, so a step's result is
+// that of solve10 bit for bit.  What it saves is lanes: solve10's half-warp forms each angle
 // on 16 lanes where 5 differ, moves every entry through shared memory and
 // waits at a barrier per step; here the relabelling is register naming.
-__device__ __forceinline__ float mul_sub(float a, float b, float c, float d) {   // a b - c d
-  return __fmaf_rn(a, b, -__fmul_rn(c, d));
-}
-__device__ __forceinline__ float mul_add(float a, float b, float c, float d) {   // a b + c d
-  return __fmaf_rn(a, b, __fmul_rn(c, d));
-}
 // position of component i after a step's round-robin relabelling
 __host__ __device__ constexpr int relabel10(int i) {
   constexpr int pr[10] = {0, 2, 4, 1, 6, 3, 8, 5, 9, 7};
@@ -1601,51 +1691,61 @@ __device__ __forceinline__ void solve11(WarpSmem<LPL, V>& sm, const Solve11Plan&
 // give the inverse.  A pivot that is positive but below 1e-10 of its
 // diagonal, where the cut might act on a nearly singular direction, makes
 // the function return false and the caller takes the Jacobi solve above.
-// 11 elimination steps over a 12 x 12 working copy instead of up to 16
-// sweeps of 11 rotation steps.
+//
+// Lane r holds row r and its right-hand side in registers, its entries moved
+// one place to the left by every elimination step, so that the pivot is always
+// the first and the steps can stay a rolled loop (the kernels that solve 11
+// terms are bound by instruction fetch).  Lane k puts the pivot row, from its
+// pivot on, in shared memory, where the others read it and the back
+// substitution finds it.  Entries spread over the lanes by division and a back
+// substitution by one lane took about twice the instructions.
 template <int LPL, int V>
 __device__ __forceinline__ bool solve11_elim(WarpSmem<LPL, V>& sm, float flambda, int lane) {
   static_assert(V == 2, "the FP64 solve belongs to the 11-term variant");
+  constexpr int P = 12;
   const double damp = 1.0 + (double)flambda;
+  const int r = lane < 11 ? lane : 10;
   double* A = sm.j11.A[0];
-  for (int i = lane; i < 144; i += 32) {
-    const int r = i / 12, c = i - 12 * (i / 12);
-    double v = 0.0;
-    if (r < 11 && c < 11) {
-      const int a = r < c ? r : c, b = r < c ? c : r;
-      v = (double)sm.alpha[upk<11>(a, b)];
-      if (r == c) v = v * damp;
-    }
-    A[i] = v;
+  double a[11], b = (double)sm.beta[r];
+#pragma unroll
+  for (int c = 0; c < 11; ++c) {
+    const double v = (double)sm.alpha[r < c ? upk<11>(r, c) : upk<11>(c, r)];
+    a[c] = r == c ? v * damp : v;
   }
-  if (lane < 12) sm.b11[lane] = lane < 11 ? (double)sm.beta[lane] : 0.0;
-  __syncwarp();
+#pragma unroll 1
   for (int k = 0; k < 11; ++k) {
-    const double piv = A[k * 13];
-    if (piv == 0.0) continue;   // a zero row and column: zero step
-    if (!(piv > 1e-10 * fabs((double)sm.alpha[upk<11>(k, k)] * damp))) return false;
-    const double inv = 1.0 / piv;
-    const int m = 10 - k;       // rows / columns after k
-    for (int e = lane; e < m * m; e += 32) {
-      const int i = k + 1 + e / m, j = k + 1 + e % m;
-      A[i * 12 + j] -= A[i * 12 + k] * inv * A[k * 12 + j];
+    double* prow = A + k * P;
+    if (lane == k) {
+#pragma unroll
+      for (int j = 0; j < 11; ++j) prow[j] = a[j];
+      prow[11] = b;
     }
-    if (lane > k && lane < 11) sm.b11[lane] -= A[lane * 12 + k] * inv * sm.b11[k];
+    __syncwarp();
+    const double piv = prow[0];
+    const bool skip = piv == 0.0;   // a zero row and column: zero step
+    if (!skip && !(piv > 1e-10 * fabs((double)sm.alpha[k * 11 - (k * (k - 1)) / 2] * damp))) return false;
+    const double inv = 1.0 / piv;
+    const double t = __dmul_rn(a[0], inv);
+    if (skip) {
+#pragma unroll
+      for (int j = 1; j < 11; ++j) a[j - 1] = a[j];
+    } else {
+#pragma unroll
+      for (int j = 1; j < 11; ++j) a[j - 1] = __fma_rn(-t, prow[j], a[j]);
+      b = __fma_rn(-t, prow[11], b);
+    }
+    a[10] = 0.0;
+  }
+#pragma unroll 1
+  for (int k = 10; k >= 0; --k) {
+    const double* row = A + k * P;
+    double s = row[11];
+#pragma unroll 2
+    for (int j = k + 1; j < 11; ++j) s = __fma_rn(-row[j - k], sm.dd[j], s);
+    const double piv = row[0];
+    if (lane == 0) sm.dd[k] = piv != 0.0 ? s / piv : 0.0;
     __syncwarp();
   }
-  if (lane == 0) {
-    for (int k = 10; k >= 0; --k) {
-      const double piv = A[k * 13];
-      double x = 0.0;
-      if (piv != 0.0) {
-        double s = sm.b11[k];
-        for (int j = k + 1; j < 11; ++j) s -= A[k * 12 + j] * sm.dd[j];
-        x = s / piv;
-      }
-      sm.dd[k] = x;
-    }
-  }
-  __syncwarp();
   return true;
 }
 

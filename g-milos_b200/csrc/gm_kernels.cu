@@ -253,7 +253,7 @@ invert_kernel(const DevCfg c, const InvertArgs a) {
 template <int LPL, int V, bool SK>
 constexpr int trial_min_blocks() { return LPL == 1 ? (V != 2 && !SK ? 7 : 5) : (V == 2 ? 8 : 10); }
 template <int LPL, int V>
-constexpr int accept_min_blocks() { return 5; }
+constexpr int accept_min_blocks() { return LPL == 1 && Variant<V>::MAC ? 4 : 5; }   // MAC: shared memory
 
 // The part of the warp's shared memory the wave kernels back.  The trial half
 // touches it only up to the first 8-row tile of staged rows (the synthesis PSF
@@ -780,7 +780,7 @@ accept_kernel(const DevCfg c0, const InvertArgs a, const WaveArgs w, int wave, c
 // Synthesis (+ response functions) of one model per warp
 // (kernel_synthesis, gmilos.cu:71-84, batched).
 template <int LPL, int V>
-__global__ void __launch_bounds__(warps_per_block<LPL>() * 32)
+__global__ void __launch_bounds__(warps_per_block<LPL>() * 32, LPL == 1 ? 4 : 5)
 synth_kernel(const DevCfg c, const SynthArgs a) {
   constexpr int NT = Variant<V>::NT;
   const int WPB = warps_per_block<LPL>();
