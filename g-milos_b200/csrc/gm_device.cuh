@@ -106,6 +106,45 @@ __device__ __forceinline__ void voigt(double a, float v, float& H, float& F) {
   F = __fdividef(im, den) * 0.5f;
 }
 
+// The same approximation with the polynomials' real coefficients used: dividing
+// by (x - z)(x - conj z) = x^2 - 2 Re z x + |z|^2 leaves b_1 z + (c_0 - |z|^2
+// b_2) as the value at z, two multiply-adds a coefficient instead of four
+// (Knuth, The Art of Computer Programming 2, 4.6.4).  Half of voigt's FP64
+// work; the values differ from its at the level of double rounding, which the
+// result's rounding to float hides but for about one value in 1e8: for the
+// synthesis kernels, not for the inversion, whose trajectories would part there.
+__device__ __forceinline__ void voigt_quad(double a, float v, float& H, float& F) {
+  const double y = (double)v, r = a + a, s = __fma_rn(a, a, y * y);
+  // z = a + i v; numerator coefficients from the highest down
+  const double p[7] = {-0.564189583562615, -5.912626209773153, -30.180142196210589, -93.155580458138441,
+                       -181.928533092181549, -214.382388694706425, -122.607931777104326};
+  double b2 = p[0], b1 = __fma_rn(r, b2, p[1]);
+#pragma unroll
+  for (int k = 2; k < 6; ++k) {
+    const double t = __fma_rn(r, b1, __fma_rn(-s, b2, p[k]));
+    b2 = b1;
+    b1 = t;
+  }
+  const double ne = __fma_rn(-s, b2, p[6]);
+  const double nr = __fma_rn(b1, a, ne), ni = b1 * y;
+  const double q[8] = {1.0, 10.479857114260399, 53.992906912940207, 170.354001821091472, 348.703917719495792,
+                       457.334478783897737, 352.730625110963558, 122.60793177387535};
+  double d2 = q[0], d1 = r + q[1];
+#pragma unroll
+  for (int k = 2; k < 7; ++k) {
+    const double t = __fma_rn(r, d1, __fma_rn(-s, d2, q[k]));
+    d2 = d1;
+    d1 = t;
+  }
+  const double de = __fma_rn(-s, d2, q[7]);
+  const double dr = __fma_rn(d1, a, de), di = d1 * y;
+  const float den = (float)(dr * dr + di * di);
+  const float re = (float)(nr * dr + ni * di);
+  const float im = (float)(ni * dr - nr * di);
+  H = -__fdividef(re, den);
+  F = __fdividef(im, den) * 0.5f;
+}
+
 // --------------------------------------------------------------- state
 struct Angles {
   float cosi, sinis, sina, cosa, sinda, cosda, sindi, cosdi, cosis_2;
@@ -523,15 +562,12 @@ __device__ __noinline__ void circ_rows(WarpSmem<LPL, V>& sm, int nl, uint64_t ma
 }
 
 // --------------------------------------------------------------- synthesis
-// ME synthesis of this lane's samples (mil_sinrf.cu:27-142 with
-// mil_sinrf_kernel :334-433): Zeeman components through the Voigt
-// profiles, Unno-Rachkovsky solution, PSF, stray-light mix.
-template <int LPL, int V>
-__device__ __forceinline__ void synth_lane(const DevCfg& c, const double* m, const float (&dlv)[LPL],
-                                           int lane, Lane<LPL, V>& st, Angles& an,
-                                           float (&spec)[LPL][4], float (&pure)[LPL][4],
-                                           const float (&sl)[LPL][4], WarpSmem<LPL, V>& sm,
-                                           const double* lamp = nullptr) {
+// ME profiles of this lane's samples before any convolution (mil_sinrf.cu:27-99
+// with mil_sinrf_kernel :334-433): Zeeman components through the Voigt
+// profiles (QUAD: voigt_quad), Unno-Rachkovsky solution.
+template <int LPL, int V, bool QUAD>
+__device__ __forceinline__ void me_lane(const DevCfg& c, const double* m, const float (&dlv)[LPL], Lane<LPL, V>& st,
+                                        Angles& an, float (&spec)[LPL][4]) {
   const float CC = (float)(kPi / 180.0), CC2 = (float)((kPi / 180.0) * 2);
   const double azi = m[AZ] * (double)CC, gmr = m[GM] * (double)CC;
   float sgm, cgm;
@@ -571,7 +607,8 @@ __device__ __forceinline__ void synth_lane(const DevCfg& c, const double* m, con
       v = v - ulos;
       v = v - rnu;
       float h, f;
-      voigt(aa, v, h, f);
+      if constexpr (QUAD) voigt_quad(aa, v, h, f);
+      else voigt(aa, v, h, f);
       const float fh = wex * h, fs = wex * f * 2.f;
 #pragma unroll
       for (int gg = 0; gg < 3; ++gg) {
@@ -614,7 +651,17 @@ __device__ __forceinline__ void synth_lane(const DevCfg& c, const double* m, con
     spec[k][2] = dtiaux * (gp5 + ru * gp2);
     spec[k][3] = dtiaux * (gp6 + rv * gp2);
   }
+}
 
+// ME synthesis of this lane's samples (mil_sinrf.cu:27-142): me_lane, PSF or
+// macroturbulence, stray-light mix.
+template <int LPL, int V, bool QUAD = false>
+__device__ __forceinline__ void synth_lane(const DevCfg& c, const double* m, const float (&dlv)[LPL],
+                                           int lane, Lane<LPL, V>& st, Angles& an,
+                                           float (&spec)[LPL][4], float (&pure)[LPL][4],
+                                           const float (&sl)[LPL][4], WarpSmem<LPL, V>& sm,
+                                           const double* lamp = nullptr) {
+  me_lane<LPL, V, QUAD>(c, m, dlv, st, an, spec);
   bool mac_on = false;
   if constexpr (Variant<V>::MAC) {
 #pragma unroll
@@ -893,6 +940,15 @@ __device__ __forceinline__ void rf_rows(const DevCfg& c, const double* m, const 
   }
 }
 
+// A double as the sum of two floats.
+struct SplitFloat {
+  float hi, lo;
+};
+__device__ __forceinline__ SplitFloat split_float(double x) {
+  const float hi = (float)x;
+  return {hi, (float)(x - (double)hi)};
+}
+
 // Response function of sample l, Stokes s, slot t in the reference's layout
 // after the PSF: 10 terms (slot 7 = S0, slot 9 = alpha) or 11 terms (slot 9
 // = v_mac, slot 10 = alpha).  Stray-light scaling, alpha's RF from the
@@ -901,7 +957,7 @@ __device__ __forceinline__ void rf_rows(const DevCfg& c, const double* m, const 
 // layout slot 9 follows alpha's flag).  mac_on: the v_mac RF rows hold the
 // derivative of the macroturbulence convolution.
 template <int LPL, int V>
-__device__ __forceinline__ float gather_rf(const DevCfg& c, const WarpSmem<LPL, V>& sm, double alfa,
+__device__ __forceinline__ float gather_rf(const DevCfg& c, const WarpSmem<LPL, V>& sm, SplitFloat alfa,
                                            float asrc, float sl, int l, int s, int t, bool mac_on) {
   constexpr int NT = Variant<V>::NT;
   const int key = (NT == 10 && t == 9) ? 10 : t;
@@ -927,7 +983,9 @@ __device__ __forceinline__ float gather_rf(const DevCfg& c, const WarpSmem<LPL, 
   } else {
     v = sm.rows[rf_row(s, t)][l];
   }
-  if (c.use_slight) v = (float)((double)v * alfa);
+  // v alfa with alfa as the sum of two floats, rounded once but for 2^-48 (the
+  // small part of an infinite v is kept finite)
+  if (c.use_slight) v = fmaf(v, alfa.hi, fminf(fmaxf(v, -3e38f), 3e38f) * alfa.lo);
   return v;
 }
 

@@ -777,17 +777,44 @@ accept_kernel(const DevCfg c0, const InvertArgs a, const WaveArgs w, int wave, c
   }
 }
 
-// Synthesis (+ response functions) of one model per warp
-// (kernel_synthesis, gmilos.cu:71-84, batched).
+// The part of the warp's shared memory the synthesis kernels back: the models
+// and the staged rows, all of them or the first 8-row tile.
+template <int LPL, int V, bool RF>
+__host__ __device__ constexpr size_t synth_warp_bytes() {
+  using WS = WarpSmem<LPL, V>;
+  constexpr size_t tile = offsetof(WS, rows) + 8 * row_pitch<LPL>() * sizeof(float);
+  return (((RF ? offsetof(WS, xrows) : tile) + 15) & ~(size_t)15) - offsetof(WS, m);
+}
+template <int LPL, int V, bool RF>
+__device__ __forceinline__ WarpSmem<LPL, V>& synth_smem() {
+  using WS = WarpSmem<LPL, V>;
+  return *reinterpret_cast<WS*>(gm_dyn_smem + tap_bytes<LPL>() +
+                                (threadIdx.x >> 5) * synth_warp_bytes<LPL, V, RF>() - offsetof(WS, m));
+}
+
+// Resident blocks per SM of the synthesis kernels.  Response functions: 16
+// warps at 128 registers; 18 and 20 spill (20 000 models of 30 samples: 138 us,
+// 155 at 18).  Profiles: 262 144 models take 302, 306, 309 us at 7, 6, 8 blocks.
+constexpr int kSynthWarps = 4;
+template <int LPL, bool RF>
+constexpr int synth_blocks() { return RF ? (LPL == 1 ? 4 : 3) : (LPL == 1 ? 7 : 4); }
+
+// Synthesis with response functions, one model per warp (kernel_synthesis,
+// gmilos.cu:71-84, batched).  Bound by issue (53 % of cycles) and the pipe that
+// FP64 and its tensor cores share (47 %): 154 us for 20 000 models of 30
+// samples before the halved Voigt polynomials (voigt_quad), one resident
+// generation of blocks and the stray-light factor applied without conversions,
+// 138 now.
 template <int LPL, int V>
-__global__ void __launch_bounds__(warps_per_block<LPL>() * 32, LPL == 1 ? 4 : 5)
-synth_kernel(const DevCfg c, const SynthArgs a) {
+__global__ void __launch_bounds__(kSynthWarps * 32, synth_blocks<LPL, true>())
+synth_rf_kernel(const DevCfg c, const SynthArgs a) {
   constexpr int NT = Variant<V>::NT;
-  const int WPB = warps_per_block<LPL>();
+  constexpr int WPB = kSynthWarps;
   const int lane = threadIdx.x & 31;
   load_taps<LPL>(c);
-  WarpSmem<LPL, V>& sm = warp_smem<LPL, V>();
-  init_rows<LPL, V>(c, sm, lane);
+  WarpSmem<LPL, V>& sm = synth_smem<LPL, V, true>();
+  for (int i = lane; i < WarpSmem<LPL, V>::NR * row_pitch<LPL>(); i += 32) (&sm.rows[0][0])[i] = 0.f;
+  __syncwarp();
   const int nl = c.nl;
   float dlv[LPL];
   double dld[LPL];
@@ -816,7 +843,7 @@ synth_kernel(const DevCfg c, const SynthArgs a) {
     Lane<LPL, V> ln;
     Angles an;
     float syn[LPL][4], pure[LPL][4];
-    synth_lane<LPL, V>(c, sm.m, dlv, lane, ln, an, syn, pure, slg, sm, lamp);
+    synth_lane<LPL, V, true>(c, sm.m, dlv, lane, ln, an, syn, pure, slg, sm, lamp);
 #pragma unroll
     for (int k = 0; k < LPL; ++k) {
       const int l = lane + 32 * k;
@@ -824,21 +851,107 @@ synth_kernel(const DevCfg c, const SynthArgs a) {
 #pragma unroll
         for (int s = 0; s < 4; ++s) a.iquv[off + s * nl + l] = syn[k][s];
     }
-    if (a.rf) {
-      rf_rows<LPL, V>(c, sm.m, ln, an, lane, sm, lamp);
-      bool mac_on = false;
-      if constexpr (Variant<V>::MAC) mac_on = sm.m[MAC] > 0.0001;
-      const size_t roff = (size_t)pix * 4 * NT * nl;
+    rf_rows<LPL, V>(c, sm.m, ln, an, lane, sm, lamp);
+    const bool mac_on = sm.m[MAC] > 0.0001;
+    const SplitFloat alfa = split_float(sm.m[ALFA]);
+    const size_t roff = (size_t)pix * 4 * NT * nl;
+#pragma unroll
+    for (int k = 0; k < LPL; ++k) {
+      const int l = lane + 32 * k;
+      if (l < nl)
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+#pragma unroll
+          for (int t = 0; t < NT; ++t)
+            a.rf[roff + ((size_t)s * NT + t) * nl + l] =
+                gather_rf<LPL, V>(c, sm, alfa, pure[k][s], slg[k][s], l, s, t, mac_on);
+    }
+    __syncwarp();
+  }
+}
+
+// Profiles only, two models per warp: their eight rows share one tile of the
+// PSF's tensor-core product (one model alone left half of it empty), each
+// macroturbulent one goes through its own circular convolution.  Without the
+// response functions' code and space 28 warps fit an SM.  Bound by issue (64 %
+// of cycles; FP64 with its tensor cores 45 %, conversions and special functions
+// 33 %): 262 144 models of 30 samples 302 us, 455 with one model per warp in
+// the kernel that also forms response functions.
+template <int LPL, int V>
+__global__ void __launch_bounds__(kSynthWarps * 32, synth_blocks<LPL, false>())
+synth_kernel(const DevCfg c, const SynthArgs a) {
+  constexpr int WPB = kSynthWarps;
+  const int lane = threadIdx.x & 31;
+  load_taps<LPL>(c);
+  WarpSmem<LPL, V>& sm = synth_smem<LPL, V, false>();
+  for (int i = lane; i < 8 * row_pitch<LPL>(); i += 32) (&sm.rows[0][0])[i] = 0.f;
+  __syncwarp();
+  const int nl = c.nl;
+  float dlv[LPL];
+  double dld[LPL];
+#pragma unroll
+  for (int k = 0; k < LPL; ++k) {
+    const int l = lane + 32 * k;
+    dlv[k] = (l < nl) ? c.dl[l] : 0.f;
+    dld[k] = 0.0;
+  }
+  float slg[LPL][4];
+  if (c.use_slight && !c.slight_per_pixel) load_pixel<LPL>(c.slight, nl, lane, slg);
+  const int64_t nw = (int64_t)gridDim.x * WPB, pairs = (a.npix + 1) / 2;
+  for (int64_t w = (int64_t)blockIdx.x * WPB + (threadIdx.x >> 5); w < pairs; w += nw) {
+    const int64_t pix = 2 * w;
+    const int n = pix + 1 < a.npix ? 2 : 1;
+    {
+      // both models: 22 lanes, 11 values each (sm.m, then sm.t)
+      const int q = lane < 11 ? 0 : 1, i = lane - 11 * q;
+      if (lane < 11 * n) {
+        const int64_t at = (pix + q) * 11 + i;
+        (q ? sm.t : sm.m)[i] = a.models_f64 ? a.models_f64[at] : (double)a.models_f32[at];
+      }
+    }
+    __syncwarp();
+    uint32_t mask = 0;
+#pragma unroll 1
+    for (int q = 0; q < n; ++q) {
+      const double* m = q ? sm.t : sm.m;
+      const double* lamp = pixel_grid<LPL>(c, (unsigned long long)(pix + q), lane, dlv, dld);
+      Lane<LPL, V> ln;
+      Angles an;
+      float spec[LPL][4];
+      me_lane<LPL, V, true>(c, m, dlv, ln, an, spec);
+      const bool mac_on = m[MAC] > 0.0001;
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        float row[LPL];
+#pragma unroll
+        for (int k = 0; k < LPL; ++k) row[k] = spec[k][s];
+        put_row<LPL, V>(sm, 4 * q + s, row, nl, lane, s == 0 && c.use_psf && !mac_on);
+      }
+      if (mac_on) {
+        mac_kernels<LPL, V>(sm, nl, c.use_psf != 0, mac_offsets<LPL>(c, lamp, lane), c.lambda0, m[MAC], lane, false);
+        circ_rows<LPL, V>(sm, nl, 0xfull << (4 * q), sm.gk, lane);
+      } else if (c.use_psf) {
+        mask |= 0xfu << (4 * q);
+      }
+    }
+    __syncwarp();
+    if (mask) psf_rows<LPL, V>(sm, c, mask, mask & 0x11u, lane);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      if (q >= n) break;
+      const size_t off = (size_t)(pix + q) * 4 * nl;
+      const double alfa = (q ? sm.t : sm.m)[ALFA];
+      if (c.use_slight && c.slight_per_pixel) load_pixel<LPL>(c.slight + off, nl, lane, slg);
 #pragma unroll
       for (int k = 0; k < LPL; ++k) {
         const int l = lane + 32 * k;
         if (l < nl)
 #pragma unroll
-          for (int s = 0; s < 4; ++s)
-#pragma unroll
-            for (int t = 0; t < NT; ++t)
-              a.rf[roff + ((size_t)s * NT + t) * nl + l] =
-                  gather_rf<LPL, V>(c, sm, sm.m[ALFA], pure[k][s], slg[k][s], l, s, t, mac_on);
+          for (int s = 0; s < 4; ++s) {
+            float v = sm.rows[4 * q + s][l];
+            if (c.use_slight) v = (float)((double)v * alfa + (double)slg[k][s] * (1.0 - alfa));
+            a.iquv[off + s * nl + l] = v;
+          }
       }
     }
     __syncwarp();
@@ -1390,27 +1503,36 @@ cudaError_t launch_invert_waves(const DevCfg& cfg, const InvertArgs& a, const Wa
   return launch_waves_v<2, 2>(cfg, a, b, s, launches);
 }
 
-template <int LPL, int V>
-cudaError_t launch_synth_t(const DevCfg& cfg, const SynthArgs& a, int grid, cudaStream_t s) {
-  const size_t bytes = tap_bytes<LPL>() + sizeof(WarpSmem<LPL, V>) * warps_per_block<LPL>();
-  cudaError_t e = cudaFuncSetAttribute(synth_kernel<LPL, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)bytes);
-  if (e != cudaSuccess) return e;
-  synth_kernel<LPL, V><<<grid, warps_per_block<LPL>() * 32, bytes, s>>>(cfg, a);
+// One resident generation of blocks, or as many as the models need.
+template <int LPL, int V, bool RF>
+cudaError_t launch_synth_t(const DevCfg& cfg, const SynthArgs& a, cudaStream_t s) {
+  constexpr int warps = kSynthWarps, per_warp = RF ? 1 : 2;
+  constexpr size_t bytes = tap_bytes<LPL>() + synth_warp_bytes<LPL, V, RF>() * warps;
+  constexpr int blocks = synth_blocks<LPL, RF>();
+  static_assert((bytes + 1024) * blocks <= kSmemPerSm, "the launch bounds' blocks fit");
+  void (*kernel)(DevCfg, SynthArgs);
+  if constexpr (RF) kernel = synth_rf_kernel<LPL, V>;
+  else kernel = synth_kernel<LPL, V>;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (bytes > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return e;
+  }
+  const int64_t need = (a.npix + warps * per_warp - 1) / (warps * per_warp), most = (int64_t)blocks * sms;
+  const int grid = (int)(need < 1 ? 1 : need < most ? need : most);
+  kernel<<<grid, warps * 32, bytes, s>>>(cfg, a);
   return cudaGetLastError();
 }
 
 cudaError_t launch_synth(const DevCfg& cfg, const SynthArgs& a, cudaStream_t s) {
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int64_t need = (a.npix + warps_for_nl(cfg.nl) - 1) / warps_for_nl(cfg.nl);
-  int grid = (int)(need < (int64_t)sms * 16 ? need : (int64_t)sms * 16);
-  if (grid < 1) grid = 1;
-  // the synthesis of arbitrary models always takes the macroturbulence-capable code
+  // the synthesis of arbitrary models always takes the macroturbulence-capable
+  // code; the number of terms matters to the response functions alone
   const bool v2 = cfg.nterms == 11;
-  if (cfg.nl <= 32) return v2 ? launch_synth_t<1, 2>(cfg, a, grid, s) : launch_synth_t<1, 1>(cfg, a, grid, s);
-  return v2 ? launch_synth_t<2, 2>(cfg, a, grid, s) : launch_synth_t<2, 1>(cfg, a, grid, s);
+  if (!a.rf) return cfg.nl <= 32 ? launch_synth_t<1, 1, false>(cfg, a, s) : launch_synth_t<2, 1, false>(cfg, a, s);
+  if (cfg.nl <= 32) return v2 ? launch_synth_t<1, 2, true>(cfg, a, s) : launch_synth_t<1, 1, true>(cfg, a, s);
+  return v2 ? launch_synth_t<2, 2, true>(cfg, a, s) : launch_synth_t<2, 1, true>(cfg, a, s);
 }
 
 cudaError_t launch_synth_grid(const DevCfg& cfg, const double* models, int64_t npix,
