@@ -264,7 +264,7 @@ struct WarpSmem {
   // any row, the accept half never solves, and the response functions are
   // consumed by the normal equations before the next solve
   union {
-    float rows[NR][row_pitch<LPL>()];
+    alignas(16) float rows[NR][row_pitch<LPL>()];
     Jacobi11<S11> j11;
   };
   // the normal equations' operand rows (kX*), right after `rows` with the
@@ -355,7 +355,8 @@ __device__ __forceinline__ void psf_rows(WarpSmem<LPL, V>& sm, const DevCfg& c, 
     const float* arow = sm.rows[r];
     const bool mine = (tile >> gr) & 1u;
     const bool refl = (reflect >> r) & 1u;
-    const double ic = refl ? (double)sm.ic[r] : 0.0;
+    // a reflected row is ic - acc, another 0 + acc, as one multiply-add
+    const double ic = refl ? (double)sm.ic[r] : 0.0, sg = refl ? -1.0 : 1.0;
     float res[LPL][4][2];
 #pragma unroll
     for (int p = 0; p < LPL; ++p) {           // output columns in passes of 32
@@ -380,19 +381,18 @@ __device__ __forceinline__ void psf_rows(WarpSmem<LPL, V>& sm, const DevCfg& c, 
 #pragma unroll
       for (int q = 0; q < 4; ++q)
 #pragma unroll
-        for (int i = 0; i < 2; ++i) res[p][q][i] = (float)(refl ? ic - acc[q][i] : acc[q][i]);
+        for (int i = 0; i < 2; ++i) res[p][q][i] = (float)__fma_rn(sg, acc[q][i], ic);
     }
     __syncwarp();
     if (mine) {
 #pragma unroll
       for (int p = 0; p < LPL; ++p)
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const int m = 32 * p + 8 * q + 2 * gc + i;
-            sm.rows[r][m] = (m < nl) ? res[p][q][i] : 0.f;
-          }
+        for (int q = 0; q < 4; ++q) {
+          const int m = 32 * p + 8 * q + 2 * gc;
+          *reinterpret_cast<float2*>(&sm.rows[r][m]) =
+              make_float2(m < nl ? res[p][q][0] : 0.f, m + 1 < nl ? res[p][q][1] : 0.f);
+        }
     }
   }
   __syncwarp();
@@ -1212,6 +1212,23 @@ __device__ __forceinline__ void ne_store(const DevCfg& c, double alfa, int e, fl
   else sm.beta[e - NA] = v;
 }
 
+// The offsets of the normal equations' operand rows, one (Stokes, term) pair
+// per lane.  They depend on the free parameters and on whether
+// macroturbulence is on: without it a kernel forms them once.
+template <int LPL, int V>
+__device__ __forceinline__ void ne_rows(const DevCfg& c, bool mac_on, int lane, WarpSmem<LPL, V>& sm) {
+  constexpr int NT = Variant<V>::NT;
+  uint32_t fixmask = 0;
+#pragma unroll
+  for (int i = 0; i < 11; ++i) fixmask |= (c.fix[i] ? 1u : 0u) << i;
+  for (int i = lane; i < 48; i += 32) {
+    const int s = i / 12, t = i - 12 * s;
+    bool scaled;
+    sm.nero[s][t] = t <= NT ? jrow<LPL, V>(c, fixmask, t, s, mac_on, scaled) * row_pitch<LPL>() : 0;
+  }
+  __syncwarp();
+}
+
 // Normal equations alpha = sum_s w_s/sigma^2 J^T J and beta = sum_s w_s J^T
 // (syn - obs) / sigma^2 (covarmf, lib.cu:65-118; covarm, lib.cu:12-63 for
 // 11 terms) in FP32 with warp-level reductions, as the reference sums them
@@ -1248,15 +1265,7 @@ __device__ __forceinline__ void normal_eq(const DevCfg& c, const double* m, bool
       sm.xrows[kXRes + s][l] = valid[k] ? syn[k][s] - ob[k][s] : 0.f;
     }
   }
-  uint32_t fixmask = 0;
-#pragma unroll
-  for (int i = 0; i < 11; ++i) fixmask |= (c.fix[i] ? 1u : 0u) << i;
-  // the operand rows' offsets: one (Stokes, term) pair per lane
-  for (int i = lane; i < 48; i += 32) {
-    const int s = i / 12, t = i - 12 * s;
-    bool scaled;
-    sm.nero[s][t] = t <= NT ? jrow<LPL, V>(c, fixmask, t, s, mac_on, scaled) * row_pitch<LPL>() : 0;
-  }
+  if constexpr (V != 0) ne_rows<LPL, V>(c, mac_on, lane, sm);   // V = 0: once per kernel
   __syncwarp();
   const float2 v01 = ne_pass64<LPL, V>(c, sm, lane);
   ne_store<LPL, V>(c, alfa, 2 * lane, v01.x, sm);
@@ -1885,6 +1894,41 @@ __device__ __forceinline__ void apply_delta_check(const F& fix, const double* m,
   if (t[MAC] > 4) t[MAC] = 4;
   if (t[ALFA] < 0) t[ALFA] = 0.0;
   if (t[ALFA] > 1.0) t[ALFA] = 1.0;
+}
+
+// The same by a warp, lane i its parameter i (lane 0 alone took about 200
+// instructions of a trial's 2600).  Step limits, lower and upper bounds per
+// parameter; the field's sign change reaches the inclination by a ballot.
+static __device__ const double g_step_limit[11] = {1e300, 300, 1e300, 1e300, 1e300, 30, 30, 1e300, 1e300, 1e300, 1e300};
+static __device__ const double g_lower[11] = {1, -1e300, -20, 0.0001, 0.0001, 0, 0, 0.0001, 0.0001, 0, 0};
+static __device__ const double g_upper[11] = {2500, 5000, 20, 0.6, 10.0, 180, 180, 2.00, 2.00, 4, 1.0};
+template <int NT, typename T, typename F>
+__device__ __forceinline__ void apply_delta_warp(const F& fix, const double* m, const T* d, double* t, int lane) {
+  const int i = lane < 11 ? lane : 10;
+  const double lim = __ldg(g_step_limit + i), lo = __ldg(g_lower + i), hi = __ldg(g_upper + i);
+  const T aux0 = d[i < 9 ? i : (i == 9 ? 9 : NT - 1)];
+  uint32_t bits = 0;
+#pragma unroll
+  for (int k = 0; k < 11; ++k) bits |= (fix[k] ? 1u : 0u) << k;
+  // limits are exact in either type; an unlimited step compares with 1e300
+  double aux = (double)aux0;
+  if (i == BFLD || i == GM || i == AZ) aux = aux < -lim ? -lim : (aux > lim ? lim : aux);
+  double x = t[i];
+  if ((bits >> i) & 1u) x = m[i] - aux;
+  const bool flip = (__ballot_sync(kFull, x < 0) >> BFLD) & 1u;
+  if (flip && i == BFLD) x = -x;
+  if (flip && i == GM) x = 180.0 - x;
+  if (i == GM) {
+    if (x < 0) x = -x;
+    if (x > 180) x = 360.0 - x;
+  } else if (i == AZ) {
+    if (x < 0) x = 180 + x;
+    if (x > 180) x = x - 180.0;
+  } else {
+    if (x < lo) x = lo;
+    if (x > hi) x = hi;
+  }
+  if (lane < 11) t[lane] = x;
 }
 
 // Weak-field and centre-of-gravity estimates of B, vlos, gamma, phi

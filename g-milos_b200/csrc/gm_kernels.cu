@@ -72,6 +72,7 @@ invert_kernel(const DevCfg c, const InvertArgs a) {
   load_taps<LPL>(c);
   WarpSmem<LPL, V>& sm = warp_smem<LPL, V>();
   init_rows<LPL, V>(c, sm, lane);
+  if constexpr (V == 0) ne_rows<LPL, V>(c, false, lane, sm);
 
   const int nl = c.nl;
   float dlv[LPL];
@@ -134,10 +135,10 @@ invert_kernel(const DevCfg c, const InvertArgs a) {
             else solve10<LPL, V, false>(sm, plan, flambda, flambda * 10.f * pbf, lane);
           }
           solved = !reuse;
-          if (lane == 0) apply_delta_check<10>(c.fix, sm.m, sm.vec[reuse ? 1 : 0][0], sm.t);
+          apply_delta_warp<10>(c.fix, sm.m, sm.vec[reuse ? 1 : 0][0], sm.t, lane);
         } else {
           if (!solve11_elim<LPL, V>(sm, flambda, lane)) solve11<LPL, V>(sm, plan11, flambda, lane);
-          if (lane == 0) apply_delta_check<11>(c.fix, sm.m, sm.dd, sm.t);
+          apply_delta_warp<11>(c.fix, sm.m, sm.dd, sm.t, lane);
         }
         __syncwarp();
       }
@@ -523,13 +524,13 @@ trial_kernel(const DevCfg c0, const InvertArgs a, const WaveArgs w, int wave, co
         __syncwarp();
         if constexpr (NT == 11) {
           if (!solve11_elim<LPL, V>(sm, flambda, lane)) solve11<LPL, V>(sm, plan11, flambda, lane);
-          if (lane == 0) apply_delta_check<11>(c.fix, sm.m, sm.dd, sm.t);
+          apply_delta_warp<11>(c.fix, sm.m, sm.dd, sm.t, lane);
         } else {
           if (!reuse) {
             if (c.numerics) solve10<LPL, V, true>(sm, plan, flambda, flambda * 10.f * pbf, lane);
             else solve10<LPL, V, false>(sm, plan, flambda, flambda * 10.f * pbf, lane);
           }
-          if (lane == 0) apply_delta_check<10>(c.fix, sm.m, sm.vec[reuse ? NS - 1 : 0][0], sm.t);
+          apply_delta_warp<10>(c.fix, sm.m, sm.vec[reuse ? NS - 1 : 0][0], sm.t, lane);
         }
       }
       solved = !reuse;
@@ -717,6 +718,7 @@ accept_kernel(const DevCfg c0, const InvertArgs a, const WaveArgs w, int wave, c
     load_taps<LPL>(c0);
     init_rows<LPL, V>(c0, sm, lane);
   }
+  if constexpr (V == 0) ne_rows<LPL, V>(c0, false, lane, sm);   // a batch's grids share the free parameters
   int nl = c0.nl;
   float dlv[LPL];
   double dld[LPL];
