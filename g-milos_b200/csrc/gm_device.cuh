@@ -756,7 +756,11 @@ __device__ __forceinline__ uint32_t rf_row_mask(const DevCfg& c) {
 // of sm (rf_row); gather_rf adds S0, alpha, the stray-light scaling
 // (:191-211) and the zeros of fixed parameters
 // (FijaACeroDerivadasNoNecesarias, milosUtils.cu:243-271).
-template <int LPL, int V>
+// FOLD (one sample per lane): the I rows are reflected as they are formed, the
+// end samples taken by shuffles, instead of in a pass of its own -- 235.5 ->
+// 233.3 ms for the 1024 x 1024 cube in the accept kernel; in the fused kernel the
+// longer code costs 1 to 5 %.
+template <int LPL, int V, bool FOLD = false>
 __device__ __forceinline__ void rf_rows(const DevCfg& c, const double* m, const Lane<LPL, V>& st,
                                         const Angles& an, int lane, WarpSmem<LPL, V>& sm,
                                         const double* lamp = nullptr) {
@@ -789,6 +793,9 @@ __device__ __forceinline__ void rf_rows(const DevCfg& c, const double* m, const 
   const float muf = c.mu;
   const uint32_t mask = rf_row_mask(c);
   const int nl = c.nl;
+  bool mac_on = false;
+  if constexpr (Variant<V>::MAC) mac_on = m[MAC] > 0.0001;
+  const bool reflect = c.use_psf && !mac_on;   // I rows, before the PSF
 
 #pragma unroll
   for (int k = 0; k < LPL; ++k) {
@@ -898,14 +905,19 @@ __device__ __forceinline__ void rf_rows(const DevCfg& c, const double* m, const 
 #pragma unroll
       for (int s = 0; s < 4; ++s) {
         const int r = rf_row(s, il);
+        if (FOLD && s == 0 && reflect) {
+          // reflected about max(first, last) on the way (me_der.cu:167-176)
+          const float f0 = __shfl_sync(kFull, o[0], 0), f1 = __shfl_sync(kFull, o[0], nl - 1);
+          const float ic = f0 > f1 ? f0 : f1;
+          if (lane == 0) sm.ic[r] = ic;
+          o[0] = ic - o[0];
+        }
         if ((mask >> r) & 1u) sm.rows[r][l] = (l < nl) ? o[s] : 0.f;
       }
     }
   }
   __syncwarp();
 
-  bool mac_on = false;
-  if constexpr (Variant<V>::MAC) mac_on = m[MAC] > 0.0001;
   if (mac_on) {
     if constexpr (Variant<V>::MAC) {
       // macroturbulence (me_der.cu:117-156): the v_mac RF is the profile
@@ -923,33 +935,32 @@ __device__ __forceinline__ void rf_rows(const DevCfg& c, const double* m, const 
       circ_rows<LPL, V>(sm, nl, 0xfull << kRows, sm.gd, lane);
       circ_rows<LPL, V>(sm, nl, (uint64_t)mask, sm.gk, lane);
     }
-  } else if (c.use_psf) {
-    // reflect the I rows about max(first, last) (me_der.cu:167-176)
-    uint32_t refl = 0;
-    float icv[8];
+  } else if (reflect) {
+    const uint32_t refl = mask & 0xffu;   // the I rows
+    if constexpr (!FOLD) {
+      // reflect them about max(first, last) (me_der.cu:167-176)
+      float icv[8];
 #pragma unroll
-    for (int tt = 0; tt < 8; ++tt) {
-      const int r = rf_row(0, tt == 7 ? 8 : tt);
-      icv[tt] = 0.f;
-      if (!((mask >> r) & 1u)) continue;
-      refl |= 1u << r;
-      const float f0 = sm.rows[r][0];
-      const float f1 = sm.rows[r][nl - 1];
-      icv[tt] = f0 > f1 ? f0 : f1;
-      if (lane == 0) sm.ic[r] = icv[tt];
-    }
-    __syncwarp();   // every lane has read the end samples before any is overwritten
-#pragma unroll
-    for (int tt = 0; tt < 8; ++tt) {
-      const int r = rf_row(0, tt == 7 ? 8 : tt);
-      if (!((refl >> r) & 1u)) continue;
-#pragma unroll
-      for (int k = 0; k < LPL; ++k) {
-        const int l = lane + 32 * k;
-        if (l < nl) sm.rows[r][l] = icv[tt] - sm.rows[r][l];
+      for (int r = 0; r < 8; ++r) {
+        icv[r] = 0.f;
+        if (!((refl >> r) & 1u)) continue;
+        const float f0 = sm.rows[r][0];
+        const float f1 = sm.rows[r][nl - 1];
+        icv[r] = f0 > f1 ? f0 : f1;
+        if (lane == 0) sm.ic[r] = icv[r];
       }
+      __syncwarp();   // every lane has read the end samples before any is overwritten
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        if (!((refl >> r) & 1u)) continue;
+#pragma unroll
+        for (int k = 0; k < LPL; ++k) {
+          const int l = lane + 32 * k;
+          if (l < nl) sm.rows[r][l] = icv[r] - sm.rows[r][l];
+        }
+      }
+      __syncwarp();
     }
-    __syncwarp();
     psf_rows<LPL, V>(sm, c, mask, refl, lane);
   }
 }
@@ -1156,13 +1167,15 @@ __device__ __forceinline__ float ne_pass(const DevCfg& c, const WarpSmem<LPL, V>
 // Entries [0, 64) in one pass (the operand rows are read once): the
 // butterfly's first step leaves 32 values per lane, the remaining four
 // halve them as in warp_reduce_scatter, and lane L ends with entries 2L and
-// 2L + 1.
+// 2L + 1.  With 10 terms entry 64, the last, is summed beside them (the lane's
+// part in `last`).
 template <int LPL, int V>
-__device__ __forceinline__ float2 ne_pass64(const DevCfg& c, const WarpSmem<LPL, V>& sm, int lane) {
+__device__ __forceinline__ float2 ne_pass64(const DevCfg& c, const WarpSmem<LPL, V>& sm, int lane, float& last) {
   constexpr int NT = Variant<V>::NT;
   float acc[64];
 #pragma unroll
   for (int i = 0; i < 64; ++i) acc[i] = 0.f;
+  last = 0.f;
 #pragma unroll 1
   for (int s = 0; s < 4; ++s) {
     const float w = c.wsig[s];
@@ -1171,6 +1184,7 @@ __device__ __forceinline__ float2 ne_pass64(const DevCfg& c, const WarpSmem<LPL,
       float x[NT + 1];
       ne_operands<LPL, V>(sm.nero[s], &sm.rows[0][0], lane + 32 * k, x);
       ne_products<NT, 0>(acc, x, w, std::make_integer_sequence<int, 64>{});
+      if constexpr (ne_entries<NT>() == 65) ne_product<NT, 64>(last, x, w);
     }
   }
   // a lane keeps entries [0, 32) (lane bit 4 clear) or [32, 64) and adds
@@ -1267,11 +1281,14 @@ __device__ __forceinline__ void normal_eq(const DevCfg& c, const double* m, bool
   }
   if constexpr (V != 0) ne_rows<LPL, V>(c, mac_on, lane, sm);   // V = 0: once per kernel
   __syncwarp();
-  const float2 v01 = ne_pass64<LPL, V>(c, sm, lane);
+  float last;
+  const float2 v01 = ne_pass64<LPL, V>(c, sm, lane, last);
   ne_store<LPL, V>(c, alfa, 2 * lane, v01.x, sm);
   ne_store<LPL, V>(c, alfa, 2 * lane + 1, v01.y, sm);
   constexpr int R = NE - 64, NL = R <= 1 ? 1 : R <= 2 ? 2 : R <= 4 ? 4 : R <= 8 ? 8 : 16;
-  const float v2 = ne_pass<LPL, V, 64, NL>(c, sm, lane);
+  float v2;
+  if constexpr (R == 1) v2 = warp_sum(last);
+  else v2 = ne_pass<LPL, V, 64, NL>(c, sm, lane);
   constexpr int sh = NL == 1 ? 5 : NL == 2 ? 4 : NL == 4 ? 3 : NL == 8 ? 2 : 1;
   const int e2 = 64 + (lane >> sh);
   if ((lane & ((1 << sh) - 1)) == 0 && e2 < NE) ne_store<LPL, V>(c, alfa, e2, v2, sm);
@@ -1455,14 +1472,10 @@ __device__ __noinline__ void solve10(WarpSmem<LPL, V>& sm, const SolvePlan& pl, 
       const float m00 = blk.x, m01 = blk.y, m11 = blk.w;
       const float m10 = diag ? m01 : blk.z;
       const float b0 = vsrc[rv], b1 = vsrc[rv + 1];
-      float th;
-      if (m00 == m11) {
-        th = quarter;
-      } else {
-        const float arc = accurate ? (2.f * m01) / (m11 - m00) : __fdividef(2.f * m01, m11 - m00);
-        th = accurate ? atanf(arc) / 2.f : __fdividef(atanf(arc), 2.f);
-        th = fminf(fmaxf(th, -qclamp), qclamp);
-      }
+      const float arc = accurate ? (2.f * m01) / (m11 - m00) : __fdividef(2.f * m01, m11 - m00);
+      float th = accurate ? atanf(arc) / 2.f : __fdividef(atanf(arc), 2.f);
+      th = fminf(fmaxf(th, -qclamp), qclamp);
+      if (m00 == m11) th = quarter;
       float sn, cs;
       sincos_mode(th, &sn, &cs, accurate);
       if (diag) {
@@ -1506,15 +1519,20 @@ __device__ __noinline__ void solve10(WarpSmem<LPL, V>& sm, const SolvePlan& pl, 
   // 8, 5, 9, 7}; undoing it, component g takes pair k = g / 2's two
   // relabelled components from their lanes (shuffles; positions packed one
   // nibble per pair) and that pair's rotation, transposed.
+  // (cs, sn) y for the pair's first component is cs y0 + sn y1, for its second
+  // cs y1 - sn y0: one multiply-add of this lane's own and its partner's value.
   const int k = g < 10 ? g >> 1 : 4, base = lane - g;
-  const int y0_lane = base + (int)((0x98640u >> (4 * k)) & 0xfu);
-  const int y1_lane = base + (int)((0x75312u >> (4 * k)) & 0xfu);
   const bool second = (g & 1) != 0;
-#pragma unroll 1
+  const int l0 = base + (int)((0x98640u >> (4 * k)) & 0xfu), l1 = base + (int)((0x75312u >> (4 * k)) & 0xfu);
+  const int own = second ? l1 : l0, other = second ? l0 : l1;
+  const unsigned sign = second ? 0x80000000u : 0u;
+  const float* rcs = &sm.cs[h][0][k];
+  const float* rsn = &sm.sn[h][0][k];
+#pragma unroll 2
   for (int step = 17; step >= 0; --step) {
-    const float y0 = __shfl_sync(kFull, y, y0_lane), y1 = __shfl_sync(kFull, y, y1_lane);
-    const float cs = sm.cs[h][step][k], sn = sm.sn[h][step][k];
-    y = second ? mul_sub(cs, y1, sn, y0) : mul_add(cs, y0, sn, y1);
+    const float ya = __shfl_sync(kFull, y, own), yb = __shfl_sync(kFull, y, other);
+    const float cs = rcs[5 * step], sn = __uint_as_float(__float_as_uint(rsn[5 * step]) ^ sign);
+    y = mul_add(cs, ya, sn, yb);
   }
   if (g < 10) sm.vec[h][0][g] = y;
   __syncwarp();

@@ -770,7 +770,7 @@ accept_kernel(const DevCfg c0, const InvertArgs a, const WaveArgs w, int wave, c
     float syn[LPL][4], pure[LPL][4];
     stage_get<LPL, V>(w.stage + (size_t)pix * stage_floats<LPL>(), ln, an, syn, pure, lane);
     __syncwarp();
-    rf_rows<LPL, V>(c, sm.m, ln, an, lane, sm, lamp);
+    rf_rows<LPL, V, LPL == 1 && V == 0>(c, sm.m, ln, an, lane, sm, lamp);
     normal_eq<LPL, V>(c, sm.m, alpha_mixed, pure, slg, syn, ob, valid, lane, sm);
     constexpr int NT = Variant<V>::NT;
     for (int i = lane; i < NT * (NT + 1) / 2; i += 32) P.alpha[i] = sm.alpha[i];
