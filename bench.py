@@ -346,7 +346,7 @@ def run_engine(args):
                      "traffic": DRAM_BYTES_PER_PIXEL * P,
                      "traffic_note": "bytes per inversion (pre-pass + trial/accept waves), scaled from an ncu "
                                      "capture of a 65536-pixel inversion",
-                     "kernels": "one step = classical pre-pass + %d trial_kernel / accept_kernel launches "
+                     "kernels": "one step = classical pre-pass + %d trial / accept / solve kernel launches "
                                 "(wave-synchronous LM); achieved = algorithmic FLOPs / the step's device time"
                                 % (launches_per_step - 1),
                      "peak_source": "measured FFMA microbenchmark (gm_measure_peaks), burst",
