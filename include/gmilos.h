@@ -197,8 +197,9 @@ gm_status gm_configure(gm_ctx *ctx, const gm_config *cfg);
  * (milosUtils.cu:658).  status (optional) receives GM_PIX_* bits.
  *
  * Kernels: inversions run wave-synchronously -- per LM trial, one kernel for the
- * trials of every pixel still iterating and one for the response functions and
- * normal equations of the accepted ones, over chunks of up to 2^20 pixels
+ * trials of every pixel still iterating, one for the response functions and
+ * normal equations of the accepted ones and, in chunks of 24576 pixels and
+ * more, one that solves for the next steps (10 terms), over chunks of up to 2^20 pixels
  * whose LM state (about 4 KB per pixel at nl <= 32, 7.4 KB above) the
  * context keeps in device memory within its HBM budget.  First-step outputs
  * (gm_lm_step), in-kernel classical estimates (gm_invert_noalloc), calls of
