@@ -126,6 +126,7 @@ struct gm_ctx {
   // and its resident-block limits per samples-per-lane class
   std::string batch_key;
   cudaGraphExec_t batch_exec = nullptr;
+  std::string batch_exec_key;         // what the captured launches hold by value
   int batch_cap[2][2] = {{0, 0}, {0, 0}};
   bool batch_tuned = false;
 };
@@ -1469,6 +1470,15 @@ extern "C" gm_status gm_invert_rois(gm_ctx* ctx, const gm_roi* rois, int nroi, c
     key += std::to_string(r.npix) + ":" + std::to_string(r.nl) + ":" + std::to_string(g) + ";";
   }
   for (int c = 0; c < 2; ++c) key += "|" + std::to_string(cls[c].cfgs.size());
+  // the kernels' variant decides their resident blocks
+  key += "|v" + std::to_string(gm::kernel_variant(base, false));
+  // A replay reads the grids' configurations from the device, where every call
+  // puts them anew; what its launches took from the configuration on the host
+  // -- the number of waves, the solve's numerics, the free parameters of the
+  // operand rows and the step limits, the alpha mix -- belongs to the capture.
+  std::string exec_key = std::to_string(base.miter) + ":" + std::to_string(base.numerics) + ":" +
+                         std::to_string(base.quirks) + ":";
+  for (int i = 0; i < GM_NPAR; ++i) exec_key += base.fix[i] ? '1' : '0';
   gm_batch_stats st{};
   int64_t total = cls[0].pixels + cls[1].pixels;
   st.pixels = total;
@@ -1560,6 +1570,11 @@ extern "C" gm_status gm_invert_rois(gm_ctx* ctx, const gm_roi* rois, int nroi, c
       ctx->batch_cap[c][1] = cls[c].ba;
     }
   }
+  // a changed configuration: capture again, the tuning stays
+  if (ctx->batch_exec && exec_key != ctx->batch_exec_key) {
+    cudaGraphExecDestroy(ctx->batch_exec);
+    ctx->batch_exec = nullptr;
+  }
   int launches = 0;
   float ms = 0.f;
   if (opts->autotune && !ctx->batch_tuned) {
@@ -1609,6 +1624,7 @@ extern "C" gm_status gm_invert_rois(gm_ctx* ctx, const gm_roi* rois, int nroi, c
         ctx->batch_exec = nullptr;
         return cuda_fail(ctx, e, "ragged-batch graph capture");
       }
+      ctx->batch_exec_key = exec_key;
     } else {
       st.graph_replayed = 1;
       for (int c = 0; c < 2; ++c)

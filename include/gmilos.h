@@ -305,7 +305,9 @@ typedef struct {
 typedef struct {
     int use_graph;                /* capture the device work of a batch in a CUDA
                                      graph and replay it for later batches of the
-                                     same layout (sizes, grids) */
+                                     same layout (sizes, grids) under the same free
+                                     parameters, iteration limit and numerics; a
+                                     call that changes any of them captures anew */
     int autotune;                 /* on the first batch of a layout, time the
                                      resident-block limits of the two wave kernels
                                      (full, 3/4, 1/2) and keep the fastest */
