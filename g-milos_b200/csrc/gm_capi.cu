@@ -127,6 +127,7 @@ struct gm_ctx {
   std::string batch_key;
   cudaGraphExec_t batch_exec = nullptr;
   std::string batch_exec_key;         // what the captured launches hold by value
+  int batch_launches = 0;             // kernels in it
   int batch_cap[2][2] = {{0, 0}, {0, 0}};
   bool batch_tuned = false;
 };
@@ -1625,14 +1626,10 @@ extern "C" gm_status gm_invert_rois(gm_ctx* ctx, const gm_roi* rois, int nroi, c
         return cuda_fail(ctx, e, "ragged-batch graph capture");
       }
       ctx->batch_exec_key = exec_key;
+      ctx->batch_launches = launches;
     } else {
       st.graph_replayed = 1;
-      for (int c = 0; c < 2; ++c)
-        if (cls[c].pixels) {
-          const int waves = 1 + (cls[c].cfgs[0].miter > 1 ? cls[c].cfgs[0].miter : 1);
-          const int64_t ch = cls[c].wb.chunk;
-          launches += (int)((cls[c].pixels + ch - 1) / ch) * (2 * waves - 1) + 1;
-        }
+      launches = ctx->batch_launches;
     }
     e = cudaEventRecord(ctx->ev0, s);
     if (e == cudaSuccess) e = cudaGraphLaunch(ctx->batch_exec, s);

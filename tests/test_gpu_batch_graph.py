@@ -73,3 +73,18 @@ def test_reconfigured_batches_equal_direct_calls(engine, rois, change):
             same(got, w)
             if replay:
                 assert st["graph_replayed"] == 1
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(init=VMAC), dict(fix=(1,) * 11, init=VMAC)], ids=["ten", "vmac", "eleven"])
+@pytest.mark.parametrize("some", [(0, 1, 2), (1, 2), (2,)])
+def test_a_replay_reports_the_launches_it_runs(engine, rois, kw, some):
+    engine.configure(config(**kw))
+    part = [rois[i] for i in some]
+    counts = []
+    for use_graph in (False, True, True):
+        _, st = batch.invert_rois(engine, part, psf_for, use_graph=use_graph)
+        counts.append(st["launches"])
+        assert engine.stats()["kernel_launches"] == st["launches"]
+    assert st["graph_replayed"] == 1
+    # every wave has a trial kernel, all but the last an accept kernel, and a class a pre-pass
+    assert counts[0] == counts[1] == counts[2] >= (1 + 2 * 13 - 1) * (1 if len(some) == 1 else 2)
