@@ -1708,7 +1708,10 @@ void gm_mlp_train_defaults(gm_mlp_train_opts* o) {
 }  // extern "C"
 
 // Training and gradients: the data staged onto the device when they are in
-// host memory, then the training driver on the context's stream.
+// host memory, then the training driver on the context's stream.  The calls
+// take no stream, so data in device memory may still be on its way there on the
+// default stream: the context's stream, which does not wait for that one by
+// itself, is made to.
 static gm_status mlp_train_impl(gm_ctx* ctx, gm_mlp* net, const float* iquv, const double* truth, int64_t n,
                                 const gm_mlp_train_opts* o, float* loss, gm_mlp* grads, bool grads_only) {
   if (!ctx || !net || !iquv || !truth || n <= 0) return ctx ? fail(ctx, GM_ERR_INVALID, "bad argument") : GM_ERR_INVALID;
@@ -1720,6 +1723,9 @@ static gm_status mlp_train_impl(gm_ctx* ctx, gm_mlp* net, const float* iquv, con
   const int nl = net->nl;
   Arg a_in, a_t;
   gm_status st;
+  cudaError_t e = cudaEventRecord(ctx->evx0, cudaStreamLegacy);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(s, ctx->evx0, 0);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "training data");
   if ((st = stage_in(ctx, "mlp_iquv", iquv, sizeof(float) * 4 * (size_t)nl * n, &a_in, s)) != GM_OK) return st;
   if ((st = stage_in(ctx, "mlp_truth", truth, sizeof(double) * 11 * (size_t)n, &a_t, s)) != GM_OK) return st;
   gm_mlp_train_opts def;
@@ -1748,8 +1754,7 @@ static gm_status mlp_train_impl(gm_ctx* ctx, gm_mlp* net, const float* iquv, con
     if ((st = ensure_buf(ctx, "mlp_ws", need, &ws)) != GM_OK) return st;
   }
   ctx->call_params.reset();
-  cudaError_t e =
-      gm::mlp::train(net, ta, ctx->call_net, ws, need, loss, grads, ctx->mlp_err, s, &why);
+  e = gm::mlp::train(net, ta, ctx->call_net, ws, need, loss, grads, ctx->mlp_err, s, &why);
   if (need > kKeepBytes) drop_buf(ctx, "mlp_ws");
   if (e == cudaErrorInvalidValue && why) return fail(ctx, GM_ERR_INVALID, why);
   if (e != cudaSuccess) return cuda_fail(ctx, e, why ? why : "training");
