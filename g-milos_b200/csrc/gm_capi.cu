@@ -1755,6 +1755,9 @@ static gm_status mlp_train_impl(gm_ctx* ctx, gm_mlp* net, const float* iquv, con
   }
   ctx->call_params.reset();
   e = gm::mlp::train(net, ta, ctx->call_net, ws, need, loss, grads, ctx->mlp_err, s, &why);
+  // what a call that failed has launched still uses the caller's data, the
+  // network's device copy and the workspace
+  if (e != cudaSuccess) cudaStreamSynchronize(s);
   if (need > kKeepBytes) drop_buf(ctx, "mlp_ws");
   if (e == cudaErrorInvalidValue && why) return fail(ctx, GM_ERR_INVALID, why);
   if (e != cudaSuccess) return cuda_fail(ctx, e, why ? why : "training");
@@ -1816,16 +1819,17 @@ gm_status gm_mlp_predict(gm_ctx* ctx, const gm_mlp* net, const float* iquv, int6
   if (e == cudaSuccess)
     e = gm::mlp::predict(ctx->call_net, (const float*)a_in.dev, n, nl, ctx->cfg.init_model, fix,
                          (double*)a_out.dev, ctx->mlp_err, s);
-  if (e == cudaSuccess && (st = copy_back(ctx, a_out, s)) != GM_OK) {
+  st = e == cudaSuccess ? copy_back(ctx, a_out, s) : cuda_fail(ctx, e, "learned initial guess");
+  if (st == GM_OK) {
+    e = cudaMemcpyAsync(ctx->mlp_err_host, ctx->mlp_err, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (e != cudaSuccess) st = cuda_fail(ctx, e, "learned initial guess");
+  }
+  // also after an error: the next call may load another network on another stream
+  e = cudaStreamSynchronize(s);
+  if (st == GM_OK && e != cudaSuccess) st = cuda_fail(ctx, e, "learned initial guess");
+  if (st != GM_OK) {
     ctx->call_params.reset();
     return st;
-  }
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(ctx->mlp_err_host, ctx->mlp_err, sizeof(int), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) {
-    ctx->call_params.reset();
-    return cuda_fail(ctx, e, "learned initial guess");
   }
   return *ctx->mlp_err_host ? learned_check(ctx) : GM_OK;
 }

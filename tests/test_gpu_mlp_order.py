@@ -1,5 +1,9 @@
-"""Training data that the default stream is still writing: gm_mlp_train and
-gm_mlp_gradients, which run on the context's stream, take it as it will be."""
+"""The order of the learned guess' calls.  Training data that the default
+stream is still writing: gm_mlp_train and gm_mlp_gradients, which run on the
+context's stream, take it as it will be.  The network that gm_mlp_predict keeps
+on the device: edited in place, exchanged for another of the same grid, trained
+or differentiated between two calls, on changing streams, every call gives what
+a context of its own gives."""
 import numpy as np
 import pytest
 
@@ -45,3 +49,44 @@ def test_training_waits_for_the_default_stream(nl, rows):
         l2, g2 = e.mlp_gradients(want, a[:512], b[:512])
         for k, v in g1.arrays().items():
             np.testing.assert_array_equal(g2.arrays()[k], v, err_msg=k)
+
+
+def test_predictions_follow_the_network():
+    torch = pytest.importorskip("torch")
+    nl, n = 30, 5000
+    lam, _ = H.grid(nl)
+    l0, _ = H.fe_line()
+    rng = np.random.default_rng(3)
+    obs = rng.normal(0.4, 0.2, (n, 4, nl)).astype(np.float32)
+    truth = H.truth_models(n, rng)
+    dev = torch.from_numpy(obs).cuda()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    cfg = G.make_config(lam, l0, ZG, init=H.GUESS)
+
+    def alone(net):
+        with G.Engine(0) as e:
+            e.configure(cfg)
+            return e.mlp_predict(net, obs)
+
+    def on_stream(e, net, k):
+        out = torch.empty((n, G.NPAR), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        G._check(G.lib().gm_mlp_predict(e._ctx, G.C.byref(net), G._ptr(dev), n, G._ptr(out),
+                                        G.C.c_void_p(streams[k].cuda_stream)), e._ctx)
+        return out.cpu().numpy()
+
+    a, b = H.random_net(1, nl), H.random_net(2, nl)
+    with G.Engine(0) as e:
+        e.configure(cfg)
+        for net in (a, b, a):
+            np.testing.assert_array_equal(e.mlp_predict(net, obs), alone(net))
+        a.arrays()["b3"][3] += 0.25
+        np.testing.assert_array_equal(e.mlp_predict(a, obs), alone(a))
+        e.mlp_gradients(b, obs[:256], truth[:256])
+        np.testing.assert_array_equal(e.mlp_predict(a, obs), alone(a))
+        e.mlp_train(b, obs, truth, epochs=1, batch=512)
+        for net in (a, b):
+            np.testing.assert_array_equal(e.mlp_predict(net, obs), alone(net))
+        for k, net in enumerate((a, b, a, b)):
+            np.testing.assert_array_equal(on_stream(e, net, (k // 2) & 1), alone(net))
