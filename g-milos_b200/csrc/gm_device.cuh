@@ -1822,7 +1822,10 @@ __device__ __forceinline__ bool solve11_elim(WarpSmem<LPL, V>& sm, float flambda
     __syncwarp();
     const double piv = prow[0];
     const bool skip = piv == 0.0;   // a zero row and column: zero step
-    if (!skip && !(piv > 1e-10 * fabs((double)sm.alpha[k * 11 - (k * (k - 1)) / 2] * damp))) return false;
+    if (!skip && !(piv > 1e-10 * fabs((double)sm.alpha[k * 11 - (k * (k - 1)) / 2] * damp))) {
+      __syncwarp();   // every lane has read the pivot row: solve11 fills the matrix anew
+      return false;
+    }
     const double inv = 1.0 / piv;
     const double t = __dmul_rn(a[0], inv);
     if (skip) {
