@@ -965,15 +965,6 @@ __device__ __forceinline__ void rf_rows(const DevCfg& c, const double* m, const 
   }
 }
 
-// A double as the sum of two floats.
-struct SplitFloat {
-  float hi, lo;
-};
-__device__ __forceinline__ SplitFloat split_float(double x) {
-  const float hi = (float)x;
-  return {hi, (float)(x - (double)hi)};
-}
-
 // Response function of sample l, Stokes s, slot t in the reference's layout
 // after the PSF: 10 terms (slot 7 = S0, slot 9 = alpha) or 11 terms (slot 9
 // = v_mac, slot 10 = alpha).  Stray-light scaling, alpha's RF from the
@@ -982,7 +973,7 @@ __device__ __forceinline__ SplitFloat split_float(double x) {
 // layout slot 9 follows alpha's flag).  mac_on: the v_mac RF rows hold the
 // derivative of the macroturbulence convolution.
 template <int LPL, int V>
-__device__ __forceinline__ float gather_rf(const DevCfg& c, const WarpSmem<LPL, V>& sm, SplitFloat alfa,
+__device__ __forceinline__ float gather_rf(const DevCfg& c, const WarpSmem<LPL, V>& sm, double alfa,
                                            float asrc, float sl, int l, int s, int t, bool mac_on) {
   constexpr int NT = Variant<V>::NT;
   const int key = (NT == 10 && t == 9) ? 10 : t;
@@ -1008,9 +999,7 @@ __device__ __forceinline__ float gather_rf(const DevCfg& c, const WarpSmem<LPL, 
   } else {
     v = sm.rows[rf_row(s, t)][l];
   }
-  // v alfa with alfa as the sum of two floats, rounded once but for 2^-48 (the
-  // small part of an infinite v is kept finite)
-  if (c.use_slight) v = fmaf(v, alfa.hi, fminf(fmaxf(v, -3e38f), 3e38f) * alfa.lo);
+  if (c.use_slight) v = (float)((double)v * alfa);
   return v;
 }
 

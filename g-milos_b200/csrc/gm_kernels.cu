@@ -795,8 +795,8 @@ __device__ __forceinline__ WarpSmem<LPL, V>& synth_smem() {
 }
 
 // Resident blocks per SM of the synthesis kernels.  Response functions: 16
-// warps at 128 registers; 18 and 20 spill (20 000 models of 30 samples: 138 us,
-// 155 at 18).  Profiles: 262 144 models take 302, 306, 309 us at 7, 6, 8 blocks.
+// warps at 128 registers; 18 and 20 spill (20 000 models of 30 samples: 147 us,
+// 155 to 163 at 18 and 20).  Profiles: 262 144 models take 302, 306, 309 us at 7, 6, 8 blocks.
 constexpr int kSynthWarps = 4;
 template <int LPL, bool RF>
 constexpr int synth_blocks() { return RF ? (LPL == 1 ? 4 : 3) : (LPL == 1 ? 7 : 4); }
@@ -804,9 +804,9 @@ constexpr int synth_blocks() { return RF ? (LPL == 1 ? 4 : 3) : (LPL == 1 ? 7 : 
 // Synthesis with response functions, one model per warp (kernel_synthesis,
 // gmilos.cu:71-84, batched).  Bound by issue (53 % of cycles) and the pipe that
 // FP64 and its tensor cores share (47 %): 154 us for 20 000 models of 30
-// samples before the halved Voigt polynomials (voigt_quad), one resident
-// generation of blocks and the stray-light factor applied without conversions,
-// 138 now.
+// samples before the halved Voigt polynomials (voigt_quad) and one resident
+// generation of blocks, 147 now.  (With the filling factor as the sum of two
+// floats, which saves two conversions a value but keeps 48 of its 53 bits, 138.)
 template <int LPL, int V>
 __global__ void __launch_bounds__(kSynthWarps * 32, synth_blocks<LPL, true>())
 synth_rf_kernel(const DevCfg c, const SynthArgs a) {
@@ -855,7 +855,7 @@ synth_rf_kernel(const DevCfg c, const SynthArgs a) {
     }
     rf_rows<LPL, V>(c, sm.m, ln, an, lane, sm, lamp);
     const bool mac_on = sm.m[MAC] > 0.0001;
-    const SplitFloat alfa = split_float(sm.m[ALFA]);
+    const double alfa = sm.m[ALFA];
     const size_t roff = (size_t)pix * 4 * NT * nl;
 #pragma unroll
     for (int k = 0; k < LPL; ++k) {
