@@ -872,16 +872,17 @@ synth_rf_kernel(const DevCfg c, const SynthArgs a) {
   }
 }
 
-// Profiles only, two models per warp: their eight rows share one tile of the
-// PSF's tensor-core product (one model alone left half of it empty), each
-// macroturbulent one goes through its own circular convolution.  Without the
+// Profiles only, `per` models per warp: the eight rows of two share one tile of
+// the PSF's tensor-core product (one model alone leaves half of it empty), each
+// macroturbulent one goes through its own circular convolution; calls too small to
+// fill the SMs take one (synth_single).  Without the
 // response functions' code and space 28 warps fit an SM.  Bound by issue (64 %
 // of cycles; FP64 with its tensor cores 45 %, conversions and special functions
 // 33 %): 262 144 models of 30 samples 302 us, 455 with one model per warp in
 // the kernel that also forms response functions.
 template <int LPL, int V>
 __global__ void __launch_bounds__(kSynthWarps * 32, synth_blocks<LPL, false>())
-synth_kernel(const DevCfg c, const SynthArgs a) {
+synth_kernel(const DevCfg c, const SynthArgs a, int per) {
   constexpr int WPB = kSynthWarps;
   const int lane = threadIdx.x & 31;
   load_taps<LPL>(c);
@@ -899,12 +900,12 @@ synth_kernel(const DevCfg c, const SynthArgs a) {
   }
   float slg[LPL][4];
   if (c.use_slight && !c.slight_per_pixel) load_pixel<LPL>(c.slight, nl, lane, slg);
-  const int64_t nw = (int64_t)gridDim.x * WPB, pairs = (a.npix + 1) / 2;
-  for (int64_t w = (int64_t)blockIdx.x * WPB + (threadIdx.x >> 5); w < pairs; w += nw) {
-    const int64_t pix = 2 * w;
-    const int n = pix + 1 < a.npix ? 2 : 1;
+  const int64_t nw = (int64_t)gridDim.x * WPB;
+  int64_t pix = per * ((int64_t)blockIdx.x * WPB + (threadIdx.x >> 5));
+  for (; pix < a.npix; pix += per * nw) {
+    const int n = pix + per <= a.npix ? per : 1;
     {
-      // both models: 22 lanes, 11 values each (sm.m, then sm.t)
+      // the models, 11 lanes each (sm.m, then sm.t)
       const int q = lane < 11 ? 0 : 1, i = lane - 11 * q;
       if (lane < 11 * n) {
         const int64_t at = (pix + q) * 11 + i;
@@ -1505,26 +1506,40 @@ cudaError_t launch_invert_waves(const DevCfg& cfg, const InvertArgs& a, const Wa
   return launch_waves_v<2, 2>(cfg, a, b, s, launches);
 }
 
+// Models per warp and SM up to which a warp of the profile kernel takes one
+// model: its pair of models is a chain twice as long, and saves only where warps
+// wait for issue or for the FP64 pipe.  30 samples with a PSF, one model a warp
+// against two: 19.9 and 21.4 us at 592 models, 21.6 and 22.1 at 2368, 23.5 and
+// 22.7 at 3100; 45 samples: 21.7 and 23.6 at 592, 23.9 and 24.9 at 1776, 25.9 and
+// 24.9 at 2368 (without a PSF the two cross later or not at all up to 6000
+// models, within 4 %).
+template <int LPL>
+constexpr int synth_single() { return LPL == 1 ? 16 : 12; }
+
 // One resident generation of blocks, or as many as the models need.
 template <int LPL, int V, bool RF>
 cudaError_t launch_synth_t(const DevCfg& cfg, const SynthArgs& a, cudaStream_t s) {
-  constexpr int warps = kSynthWarps, per_warp = RF ? 1 : 2;
+  constexpr int warps = kSynthWarps;
   constexpr size_t bytes = tap_bytes<LPL>() + synth_warp_bytes<LPL, V, RF>() * warps;
   constexpr int blocks = synth_blocks<LPL, RF>();
   static_assert((bytes + 1024) * blocks <= kSmemPerSm, "the launch bounds' blocks fit");
-  void (*kernel)(DevCfg, SynthArgs);
-  if constexpr (RF) kernel = synth_rf_kernel<LPL, V>;
-  else kernel = synth_kernel<LPL, V>;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (bytes > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    cudaError_t e;
+    if constexpr (RF)
+      e = cudaFuncSetAttribute(synth_rf_kernel<LPL, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    else
+      e = cudaFuncSetAttribute(synth_kernel<LPL, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return e;
   }
-  const int64_t need = (a.npix + warps * per_warp - 1) / (warps * per_warp), most = (int64_t)blocks * sms;
+  const int64_t most = (int64_t)blocks * sms;
+  const int per = RF || a.npix <= (int64_t)synth_single<LPL>() * sms ? 1 : 2;
+  const int64_t need = (a.npix + warps * per - 1) / (warps * per);
   const int grid = (int)(need < 1 ? 1 : need < most ? need : most);
-  kernel<<<grid, warps * 32, bytes, s>>>(cfg, a);
+  if constexpr (RF) synth_rf_kernel<LPL, V><<<grid, warps * 32, bytes, s>>>(cfg, a);
+  else synth_kernel<LPL, V><<<grid, warps * 32, bytes, s>>>(cfg, a, per);
   return cudaGetLastError();
 }
 
