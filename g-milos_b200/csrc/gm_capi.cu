@@ -1520,14 +1520,14 @@ extern "C" gm_status gm_invert_rois(gm_ctx* ctx, const gm_roi* rois, int nroi, c
     k.grid = (uint16_t*)q;
     if ((stt = ensure_buf(ctx, p + "off", sizeof(uint64_t) * P, &q)) != GM_OK) return stt;
     k.off = (uint64_t*)q;
-    gm::waves_mg_occupancy(k.cfgs[0], &k.bt, &k.ba);
-    if (k.bt < 1 || k.ba < 1) return fail(ctx, GM_ERR_CUDA, "ragged-batch kernels cannot be resident");
   }
   for (int c = 0; c < 2; ++c) {
     BatchClass& k = cls[c];
     if (!k.pixels) continue;
     const int64_t chunk = wave_chunk_for(ctx, k.cfgs[0], need, k.pixels, 2);
     if (!chunk) return fail(ctx, GM_ERR_NOMEM, "the batch's wave state does not fit the HBM budget");
+    gm::waves_mg_occupancy(k.cfgs[0], chunk, &k.bt, &k.ba);
+    if (k.bt < 1 || k.ba < 1) return fail(ctx, GM_ERR_CUDA, "ragged-batch kernels cannot be resident");
     if ((stt = wave_buffers(ctx, c ? "rg1_waves" : "rg0_waves", k.cfgs[0], chunk, &k.wb)) != GM_OK) return stt;
     key += "|" + std::to_string(chunk) + "@" + std::to_string((uintptr_t)k.wb.w.state) + "/" +
            std::to_string((uintptr_t)k.in);

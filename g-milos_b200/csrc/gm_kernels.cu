@@ -1,5 +1,6 @@
 // gm_kernels.cu -- persistent LM inversion kernel, synthesis kernels.
 #include <cstddef>
+#include <type_traits>
 
 #include "gm_kernels.cuh"
 
@@ -1398,6 +1399,13 @@ cudaError_t run_waves(const DevCfg& dc, const InvertArgs& c, const WaveBuffers& 
 constexpr int64_t kSolveApartMin = 24576;
 template <int V>
 constexpr bool solve_apart(int64_t n) { return V != 2 && n >= kSolveApartMin; }
+// Ragged batches, whose launch count nothing relies on, take it from where it
+// pays.  Early stop, PSF: 2.06 ms against 1.67 without the solve kernel at 256
+// pixels of 30 samples, 3.42 against 3.30 at 8100, 4.15 and 4.12 at 12 544, 6.17
+// against 6.60 at 24 336; at 45 samples 3.67 against 3.39 at 4096, 4.85 and 4.70
+// at 8100, 6.29 against 6.36 at 12 544; without a PSF even at 16 384.
+constexpr int64_t kSolveApartMinMg = 12288;
+constexpr bool solve_apart_mg(int64_t n) { return n >= kSolveApartMinMg; }
 
 template <int LPL, int V, bool SK>
 cudaError_t launch_waves_t(const DevCfg& cfg, const InvertArgs& a, const WaveBuffers& b, cudaStream_t s,
@@ -1425,11 +1433,10 @@ cudaError_t launch_waves_t(const DevCfg& cfg, const InvertArgs& a, const WaveBuf
 // Ragged batches: chunks of the batch's pixel list; profiles and fitted
 // profiles are addressed through mg.off, so only the per-pixel outputs,
 // start models and tables move with the chunk.
-template <int LPL, int V>
+template <int LPL, int V, bool SK>
 cudaError_t launch_waves_mg_t(const DevCfg& cfg, const MultiGrid& mg, const InvertArgs& a, const WaveBuffers& b,
                               int cap_t, int cap_a, cudaStream_t s, int* launches) {
   int dev = 0, sms = 0, bt = 0, ba = 0;
-  constexpr bool SK = V != 2;
   cudaError_t e = wave_occupancy<LPL, V, true, SK>(&bt, &ba);
   if (e != cudaSuccess) return e;
   if (cap_t > 0 && cap_t < bt) bt = cap_t;
@@ -1454,31 +1461,41 @@ cudaError_t launch_waves_mg_t(const DevCfg& cfg, const MultiGrid& mg, const Inve
   return cudaSuccess;
 }
 
+// Calls f with the types of a ragged batch's kernels: samples per lane,
+// variant and whether the solve kernel makes the steps of chunks of n pixels.
+template <typename F>
+cudaError_t with_mg_kernels(const DevCfg& cfg, int64_t n, F f) {
+  using std::integral_constant;
+  auto pick = [&](auto lpl, auto v) {
+    if constexpr (decltype(v)::value != 2) {
+      if (solve_apart_mg(n)) return f(lpl, v, std::true_type{});
+    }
+    return f(lpl, v, std::false_type{});
+  };
+  auto variant = [&](auto lpl) {
+    const int v = kernel_variant(cfg, false);
+    if (v == 0) return pick(lpl, integral_constant<int, 0>{});
+    if (v == 1) return pick(lpl, integral_constant<int, 1>{});
+    return pick(lpl, integral_constant<int, 2>{});
+  };
+  return cfg.nl <= 32 ? variant(integral_constant<int, 1>{}) : variant(integral_constant<int, 2>{});
+}
+
 cudaError_t launch_invert_waves_mg(const DevCfg& cfg, const MultiGrid& mg, const InvertArgs& a,
                                    const WaveBuffers& b, int cap_t, int cap_a, cudaStream_t s, int* launches) {
   if (!waves_cover(cfg, a) || !a.init_status || b.chunk < 1 || b.chunk > 0x7fffffff || cfg.lambda_per_pixel ||
       (cfg.use_slight && cfg.slight_per_pixel))
     return cudaErrorInvalidValue;
-  const int v = kernel_variant(cfg, false);
-  if (cfg.nl <= 32) {
-    if (v == 0) return launch_waves_mg_t<1, 0>(cfg, mg, a, b, cap_t, cap_a, s, launches);
-    if (v == 1) return launch_waves_mg_t<1, 1>(cfg, mg, a, b, cap_t, cap_a, s, launches);
-    return launch_waves_mg_t<1, 2>(cfg, mg, a, b, cap_t, cap_a, s, launches);
-  }
-  if (v == 0) return launch_waves_mg_t<2, 0>(cfg, mg, a, b, cap_t, cap_a, s, launches);
-  if (v == 1) return launch_waves_mg_t<2, 1>(cfg, mg, a, b, cap_t, cap_a, s, launches);
-  return launch_waves_mg_t<2, 2>(cfg, mg, a, b, cap_t, cap_a, s, launches);
+  return with_mg_kernels(cfg, a.npix < b.chunk ? a.npix : b.chunk, [&](auto lpl, auto v, auto sk) {
+    return launch_waves_mg_t<decltype(lpl)::value, decltype(v)::value, decltype(sk)::value>(cfg, mg, a, b, cap_t,
+                                                                                             cap_a, s, launches);
+  });
 }
 
-void waves_mg_occupancy(const DevCfg& cfg, int* bt, int* ba) {
-  const int v = kernel_variant(cfg, false);
-  cudaError_t e;
-  if (cfg.nl <= 32)
-    e = v == 0 ? wave_occupancy<1, 0, true, true>(bt, ba) : v == 1 ? wave_occupancy<1, 1, true, true>(bt, ba)
-                                                             : wave_occupancy<1, 2, true, false>(bt, ba);
-  else
-    e = v == 0 ? wave_occupancy<2, 0, true, true>(bt, ba) : v == 1 ? wave_occupancy<2, 1, true, true>(bt, ba)
-                                                             : wave_occupancy<2, 2, true, false>(bt, ba);
+void waves_mg_occupancy(const DevCfg& cfg, int64_t n, int* bt, int* ba) {
+  const cudaError_t e = with_mg_kernels(cfg, n, [&](auto lpl, auto v, auto sk) {
+    return wave_occupancy<decltype(lpl)::value, decltype(v)::value, true, decltype(sk)::value>(bt, ba);
+  });
   if (e != cudaSuccess) *bt = *ba = 0;
 }
 

@@ -150,8 +150,9 @@ cudaError_t launch_invert_waves_mg(const DevCfg& cfg, const MultiGrid& mg, const
                                    int* launches);
 cudaError_t launch_classical_mg(const DevCfg& cfg, const MultiGrid& mg, const float* iquv, int64_t npix,
                                 double* models, uint32_t* status, cudaStream_t s);
-// resident blocks per SM of the ragged-batch wave kernels (the autotuner's range)
-void waves_mg_occupancy(const DevCfg& cfg, int* trial_blocks, int* accept_blocks);
+// resident blocks per SM of the ragged-batch wave kernels for chunks of n pixels
+// (the autotuner's range)
+void waves_mg_occupancy(const DevCfg& cfg, int64_t n, int* trial_blocks, int* accept_blocks);
 cudaError_t launch_synth(const DevCfg& cfg, const SynthArgs& a, cudaStream_t s);
 // classical estimates: for_init false -> the classical-estimates mode
 // (S0 = B_los); true -> start models of an inversion plus status bits

@@ -88,3 +88,22 @@ def test_a_replay_reports_the_launches_it_runs(engine, rois, kw, some):
     assert st["graph_replayed"] == 1
     # every wave has a trial kernel, all but the last an accept kernel, and a class a pre-pass
     assert counts[0] == counts[1] == counts[2] >= (1 + 2 * 13 - 1) * (1 if len(some) == 1 else 2)
+
+
+def test_the_solve_kernel_of_large_batches_changes_nothing(engine, rois):
+    """A class of 12 288 pixels and more makes its steps in a kernel of its own:
+    regions alone on either side of that, in 10 terms with and without
+    macroturbulence, at one and two samples per lane, equal those in a batch
+    beyond it, bit for bit."""
+    lam45, _ = H.grid(45)
+    obs, lam = rois[0]
+    few, _ = rois[1]
+    wide = np.ascontiguousarray(np.tile(few, (50, 1, 1))[:12288])
+    for kw in (dict(), dict(init=VMAC), dict(numerics=1), dict(logclambda=1), dict(fix=(0, 1) + (0,) * 9)):
+        engine.configure(config(**kw))
+        for cube, grid in ((obs[:12288], lam), (wide, lam45)):
+            whole, large = batch.invert_rois(engine, [(cube, grid)], psf_for)
+            part, small = batch.invert_rois(engine, [(np.ascontiguousarray(cube[:12287]), grid)], psf_for)
+            assert large["launches"] == 1 + 3 * 13 - 2 and small["launches"] == 1 + 2 * 13 - 1
+            for k in KEYS:
+                np.testing.assert_array_equal(whole[0][k][:12287], part[0][k], err_msg=k)
