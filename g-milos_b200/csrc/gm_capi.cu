@@ -155,6 +155,16 @@ bool is_device_ptr(const void* p) {
   return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
 }
 
+void drop_buf(gm_ctx* ctx, const std::string& name) {
+  auto it = ctx->bufs.find(name);
+  if (it == ctx->bufs.end()) return;
+  if (it->second.p) cudaFree(it->second.p);
+  it->second = DevBuf{};
+}
+
+// The training workspace, kept between calls while it is small.
+const char* const kTrainBuf = "mlp_ws";
+
 gm_status ensure_buf(gm_ctx* ctx, const std::string& name, size_t bytes, void** out) {
   DevBuf& b = ctx->bufs[name];
   if (b.bytes < bytes) {
@@ -163,20 +173,20 @@ gm_status ensure_buf(gm_ctx* ctx, const std::string& name, size_t bytes, void** 
     b.bytes = 0;
     cudaError_t e = cudaMalloc(&b.p, bytes);
     if (e != cudaSuccess) {
+      // the training workspace makes room for others
       cudaGetLastError();
+      drop_buf(ctx, kTrainBuf);
+      e = cudaMalloc(&b.p, bytes);
+    }
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      b.p = nullptr;
       return fail(ctx, GM_ERR_NOMEM, "device allocation of " + std::to_string(bytes) + " bytes failed");
     }
     b.bytes = bytes;
   }
   *out = b.p;
   return GM_OK;
-}
-
-void drop_buf(gm_ctx* ctx, const std::string& name) {
-  auto it = ctx->bufs.find(name);
-  if (it == ctx->bufs.end()) return;
-  if (it->second.p) cudaFree(it->second.p);
-  ctx->bufs.erase(it);
 }
 
 // A host- or device-side argument staged onto the device.
@@ -1751,14 +1761,14 @@ static gm_status mlp_train_impl(gm_ctx* ctx, gm_mlp* net, const float* iquv, con
   size_t need = 0;
   if (batch > 0 && batch % gm::mlp::kTile == 0 && n >= batch && n <= (int64_t)1 << 31) {
     need = gm::mlp::train_bytes(n, batch);
-    if ((st = ensure_buf(ctx, "mlp_ws", need, &ws)) != GM_OK) return st;
+    if ((st = ensure_buf(ctx, kTrainBuf, need, &ws)) != GM_OK) return st;
   }
   ctx->call_params.reset();
   e = gm::mlp::train(net, ta, ctx->call_net, ws, need, loss, grads, ctx->mlp_err, s, &why);
   // what a call that failed has launched still uses the caller's data, the
   // network's device copy and the workspace
   if (e != cudaSuccess) cudaStreamSynchronize(s);
-  if (need > kKeepBytes) drop_buf(ctx, "mlp_ws");
+  if (need > kKeepBytes) drop_buf(ctx, kTrainBuf);
   if (e == cudaErrorInvalidValue && why) return fail(ctx, GM_ERR_INVALID, why);
   if (e != cudaSuccess) return cuda_fail(ctx, e, why ? why : "training");
   return GM_OK;

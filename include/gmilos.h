@@ -446,7 +446,10 @@ void gm_mlp_train_defaults(gm_mlp_train_opts *o);
  * FP32 parameters).  An untrained net (steps == 0) first takes its
  * standardisation from the data.  loss_per_epoch (optional, [epochs]): mean
  * squared error of the standardised outputs over each epoch.  n must be at
- * least one batch.  Profiles in device memory must start on a 16-byte
+ * least one batch.  Device memory beside the data (about 3.5 KB a batch row,
+ * 68 bytes a pixel and 6 MB) is taken outside the context's HBM budget; up to
+ * 256 MB of it stays with the context for the next call, until gm_destroy or an
+ * allocation of the context that finds no room without it.  Profiles in device memory must start on a 16-byte
  * boundary (the kernels read them in 16-byte vectors), as must the cube of
  * an inversion that starts from the learned guess (GM_INIT_LEARNED);
  * otherwise the call fails before the network runs (GM_ERR_INVALID here and

@@ -90,3 +90,29 @@ def test_predictions_follow_the_network():
             np.testing.assert_array_equal(e.mlp_predict(net, obs), alone(net))
         for k, net in enumerate((a, b, a, b)):
             np.testing.assert_array_equal(on_stream(e, net, (k // 2) & 1), alone(net))
+
+
+def test_the_training_workspace_makes_room():
+    """The workspace that stays with the context is given back when another
+    allocation fails (one of 352 GB here, refused at once), and is made again by
+    the next training call."""
+    torch = pytest.importorskip("torch")
+    nl, n = 30, 16384
+    lam, _ = H.grid(nl)
+    l0, _ = H.fe_line()
+    rng = np.random.default_rng(8)
+    truth = torch.from_numpy(H.truth_models(n, rng)).cuda()
+    obs = torch.from_numpy(rng.normal(0.4, 0.2, (n, 4, nl)).astype(np.float32)).cuda()
+    model = np.zeros((1, 11))
+    out = np.zeros((1, 4, nl), np.float32)
+    with G.Engine(0) as e:
+        e.configure(G.make_config(lam, l0, ZG, init=H.GUESS))
+        net = G.mlp_new(nl, 5)
+        e.mlp_train(net, obs, truth, epochs=1, batch=n)
+        kept = torch.cuda.mem_get_info()[0]
+        with pytest.raises(G.GmError):
+            G._check(G.lib().gm_synthesize_f64(e._ctx, G._ptr(model), 4_000_000_000, G._ptr(out), None, None), e._ctx)
+        # 3.5 KB a row of the batch
+        assert torch.cuda.mem_get_info()[0] - kept > 3000 * n
+        loss = e.mlp_train(net, obs, truth, epochs=1, batch=n)
+        assert np.isfinite(loss).all()
