@@ -110,9 +110,12 @@ __device__ __forceinline__ void voigt(double a, float v, float& H, float& F) {
 // by (x - z)(x - conj z) = x^2 - 2 Re z x + |z|^2 leaves b_1 z + (c_0 - |z|^2
 // b_2) as the value at z, two multiply-adds a coefficient instead of four
 // (Knuth, The Art of Computer Programming 2, 4.6.4).  Half of voigt's FP64
-// work; the values differ from its at the level of double rounding, which the
-// result's rounding to float hides but for about one value in 1e8: for the
-// synthesis kernels, not for the inversion, whose trajectories would part there.
+// work.  Against 128-bit arithmetic (|v| <= 30, 4e6 draws) the real part rounds to
+// another float for 0.8e-6 of the arguments at damping 0 to 0.5 and 1.8e-6 at 1e-4 to
+// 0.05, voigt's for 1.3e-6 and 2.5e-6, and where a = 0 leaves the real part to
+// cancellation its error is a quarter of voigt's.  The two differ for about 2e-6 of
+// the arguments: this one is for the synthesis kernels, not for the inversion,
+// whose trajectories would part there.
 __device__ __forceinline__ void voigt_quad(double a, float v, float& H, float& F) {
   const double y = (double)v, r = a + a, s = __fma_rn(a, a, y * y);
   // z = a + i v; numerator coefficients from the highest down
@@ -1844,21 +1847,10 @@ __device__ __forceinline__ bool solve11_elim(WarpSmem<LPL, V>& sm, float flambda
 // model -= delta on free parameters with the reference's step limits
 // (AplicaDeltaf, milosUtils.cu:93-159, float delta; AplicaDelta, :30-91,
 // double delta for 11 terms), then range checks (check, :160-238).  The
-// filling factor's step is slot 9 of 10 or slot 10 of 11.
-// fix: the free-parameter flags, an array or a FixMask.
-struct FixMask {
-  uint32_t bits;
-  __device__ __forceinline__ bool operator[](int i) const { return (bits >> i) & 1u; }
-};
-__device__ __forceinline__ FixMask fix_mask(const DevCfg& c) {
-  FixMask f{0u};
-#pragma unroll
-  for (int i = 0; i < 11; ++i) f.bits |= (c.fix[i] ? 1u : 0u) << i;
-  return f;
-}
-template <int NT, typename T, typename F>
-__device__ __forceinline__ void apply_delta_check(const F& fix, const double* m, const T* d, double* t) {
-  T aux;
+// filling factor's step is slot 9 of 10 or slot 10 of 11.  By one thread, for
+// the 10 terms of the solve kernel.
+__device__ __forceinline__ void apply_delta_check(const int (&fix)[11], const double* m, const float* d, double* t) {
+  float aux;
   if (fix[ETA0]) t[ETA0] = m[ETA0] - d[0];
   if (fix[BFLD]) {
     aux = d[1];
@@ -1881,7 +1873,7 @@ __device__ __forceinline__ void apply_delta_check(const F& fix, const double* m,
   if (fix[S0]) t[S0] = m[S0] - d[7];
   if (fix[S1]) t[S1] = m[S1] - d[8];
   if (fix[MAC]) t[MAC] = m[MAC] - d[9];
-  if (fix[ALFA]) t[ALFA] = m[ALFA] - d[NT == 11 ? 10 : 9];
+  if (fix[ALFA]) t[ALFA] = m[ALFA] - d[9];
   if (t[BFLD] < 0) { t[BFLD] = -t[BFLD]; t[GM] = 180.0 - t[GM]; }
   if (t[BFLD] > 5000) t[BFLD] = 5000;
   if (t[GM] < 0) t[GM] = -t[GM];
@@ -1912,8 +1904,9 @@ __device__ __forceinline__ void apply_delta_check(const F& fix, const double* m,
 static __device__ const double g_step_limit[11] = {1e300, 300, 1e300, 1e300, 1e300, 30, 30, 1e300, 1e300, 1e300, 1e300};
 static __device__ const double g_lower[11] = {1, -1e300, -20, 0.0001, 0.0001, 0, 0, 0.0001, 0.0001, 0, 0};
 static __device__ const double g_upper[11] = {2500, 5000, 20, 0.6, 10.0, 180, 180, 2.00, 2.00, 4, 1.0};
-template <int NT, typename T, typename F>
-__device__ __forceinline__ void apply_delta_warp(const F& fix, const double* m, const T* d, double* t, int lane) {
+template <int NT, typename T>
+__device__ __forceinline__ void apply_delta_warp(const int (&fix)[11], const double* m, const T* d, double* t,
+                                                 int lane) {
   const int i = lane < 11 ? lane : 10;
   const double lim = __ldg(g_step_limit + i), lo = __ldg(g_lower + i), hi = __ldg(g_upper + i);
   const T aux0 = d[i < 9 ? i : (i == 9 ? 9 : NT - 1)];

@@ -652,7 +652,7 @@ solve_kernel(const DevCfg c, const WaveArgs w, int wave) {
     double t[11];
 #pragma unroll
     for (int k = 0; k < 11; ++k) t[k] = P.t[k];
-    apply_delta_check<10>(c.fix, P.m, P.vnext, t);
+    apply_delta_check(c.fix, P.m, P.vnext, t);
 #pragma unroll
     for (int k = 0; k < 11; ++k) P.t[k] = t[k];
   }
@@ -699,7 +699,7 @@ solve_kernel(const DevCfg c, const WaveArgs w, int wave) {
         double t[11];
 #pragma unroll
         for (int k = 0; k < 11; ++k) t[k] = P.t[k];
-        apply_delta_check<10>(c.fix, P.m, v, t);
+        apply_delta_check(c.fix, P.m, v, t);
 #pragma unroll
         for (int k = 0; k < 11; ++k) P.t[k] = t[k];
       }

@@ -30,7 +30,6 @@
 #include <cmath>
 #include <cstring>
 #include <random>
-#include <vector>
 
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
@@ -593,7 +592,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(b)) : "memory");
 }
 
-// Producer state (warp 8, lane 0)
+// Producer state (warp 16, lane 0)
 struct Prod {
   uint32_t fph[2] = {0, 0}, eph[2] = {0, 0}, hph[2] = {0, 0};
   bool pend[2] = {false, false}, inflight[2] = {false, false};
