@@ -45,11 +45,11 @@ GUESS_VMAC = GUESS[:9] + (0.5, 1.0)
 MAXITER = 50
 
 # DRAM bytes (read + write) per pixel of one inversion (classical pre-pass
-# and every trial / accept wave), measured with ncu (dram__bytes_read.sum +
-# dram__bytes_write.sum summed over the 102 launches of an inversion) on
-# 65 536-pixel inversions of this workload with the current kernels;
-# traffic grows with the pixel count.
-DRAM_BYTES_PER_PIXEL = 206500.0
+# and every trial / accept / solve wave), measured with ncu
+# (dram__bytes_read.sum + dram__bytes_write.sum summed over the 152 launches
+# of an inversion) on a 65 536-pixel inversion of this workload; traffic grows
+# with the pixel count.
+DRAM_BYTES_PER_PIXEL = 204100.0
 
 # Algorithmic FLOPs per pixel (per-wavelength costs counted from the formulas)
 C_VOIGT, C_RTE, C_DVOIGT, C_DRTE = 100, 85, 23, 870
@@ -344,7 +344,7 @@ def run_engine(args):
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s",
                      "frac": achieved / fp32_peak if fp32_peak else None,
                      "traffic": DRAM_BYTES_PER_PIXEL * P,
-                     "traffic_note": "bytes per inversion (pre-pass + trial/accept waves), scaled from an ncu "
+                     "traffic_note": "bytes per inversion (pre-pass + trial/accept/solve waves), scaled from an ncu "
                                      "capture of a 65536-pixel inversion",
                      "kernels": "one step = classical pre-pass + %d trial / accept / solve kernel launches "
                                 "(wave-synchronous LM); achieved = algorithmic FLOPs / the step's device time"

@@ -474,9 +474,13 @@ constexpr int64_t kWaveMinChunk = 16384;
 
 // Calls (or served requests) of fewer pixels than this run the fused
 // persistent kernel under GM_KERNEL_AUTO: there the wave kernels' ~100 short
-// launches cost more than their split saves (measured on B200 at 30
-// samples: 4096 pixels with a PSF invert 1.4x faster fused, without one
-// 1.9x; the two are even at 16384 pixels with a PSF and at ~32768 without).
+// launches cost more than their split saves.  Device time, waves against
+// fused, 30 samples and 10 terms: with a PSF 2.51 and 1.72 ms at 4096 pixels,
+// 3.33 and 2.97 at 8192, 5.41 and 5.54 at 16384; without one 1.79 and 0.88,
+// 2.23 and 1.55, 3.22 and 2.78, 4.91 and 5.30 at 32768.  With macroturbulence,
+// 11 terms or 33 to 64 samples the two cross lower, between 4096 and 8192
+// pixels (45 samples with a PSF: 3.26 and 3.16 ms at 4096, 5.05 and 5.75 at
+// 8192); the one line holds for all.
 static int64_t fused_below(const gm::DevCfg& d) { return d.use_psf ? 16384 : 32768; }
 
 // Which kernels invert a call of npix pixels: the wave-synchronous kernels

@@ -796,8 +796,8 @@ __device__ __forceinline__ WarpSmem<LPL, V>& synth_smem() {
 }
 
 // Resident blocks per SM of the synthesis kernels.  Response functions: 16
-// warps at 128 registers; 18 and 20 spill (20 000 models of 30 samples: 147 us,
-// 155 to 163 at 18 and 20).  Profiles: 262 144 models take 302, 306, 309 us at 7, 6, 8 blocks.
+// warps at 128 registers; 18 and 20 spill (20 000 models of 30 samples, at the
+// time 138 us: 155 and 163).  Profiles: 262 144 models take 302, 306, 309 us at 7, 6, 8 blocks.
 constexpr int kSynthWarps = 4;
 template <int LPL, bool RF>
 constexpr int synth_blocks() { return RF ? (LPL == 1 ? 4 : 3) : (LPL == 1 ? 7 : 4); }
@@ -1389,8 +1389,8 @@ cudaError_t run_waves(const DevCfg& dc, const InvertArgs& c, const WaveBuffers& 
   return cudaGetLastError();
 }
 
-// Whether the solve kernel makes the steps of a chunk of n pixels (10 terms;
-// the results are those of the solve in the trial kernel bit for bit).  Its
+// Whether the solve kernel makes the steps of a chunk of n pixels (10 terms,
+// one grid; the results are those of the solve in the trial kernel bit for bit).  Its
 // launch pays from about 8000 pixels on: 30 samples and a PSF take 2.87 ms
 // against 2.76 with the solve in the trial kernel at 4096 pixels, 5.42
 // against 5.85 at 16 384, 9.15 against 10.53 at 32 768, 16.6 against 19.8 at
